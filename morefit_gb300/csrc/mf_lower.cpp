@@ -444,6 +444,22 @@ std::vector<char> reachable(const std::vector<Node>& ns, const std::vector<int>&
   return r;
 }
 
+// Operands of which both sin and cos are live per-event values: operand -> (sin node, cos node).
+std::map<int, std::pair<int, int>> sincos_pairs(const std::vector<Node>& ns, const std::vector<char>& live) {
+  std::map<int, int> sin_of, cos_of;
+  std::map<int, std::pair<int, int>> r;
+  for (size_t i = 0; i < ns.size(); i++) {
+    if (!live[i] || ns[i].uniform) continue;
+    if (ns[i].op == Op::Sin) sin_of[ns[i].a] = int(i);
+    if (ns[i].op == Op::Cos) cos_of[ns[i].a] = int(i);
+  }
+  for (auto& [a, si] : sin_of) {
+    auto c = cos_of.find(a);
+    if (c != cos_of.end()) r[a] = {si, c->second};
+  }
+  return r;
+}
+
 struct Emitter {
   const std::vector<Node>& ns;
   bool f32;  // arithmetic type float
@@ -886,6 +902,99 @@ __device__ __forceinline__ mf_dw mf_dw_shfl_xor(mf_dw a, int o) {
 }
 )CUDA";
 
+// FP32 values with a running bound of their error, for the generator's accept
+// test: the exact value of the expression lies within e of v. Every operation
+// adds to the propagated bounds of its operands the rounding of its own result
+// (kept at twice 2^-24 relative, which also covers the rounding of the bounds
+// themselves, plus 2^-126 for results that underflow); the functions' results
+// are taken as within 4 units of 2^-23 (CUDA's documented maximum errors are
+// smaller), and their slopes are bounded over the whole interval the operand
+// may lie in, or the bound is infinite where it may reach a pole or a branch.
+// The caller tests the final bound with 1% to spare.
+const char* kEfPrelude = R"CUDA(
+struct mf_ef { float v, e; };
+#define MF_EF_INF __int_as_float(0x7f800000)
+__device__ __forceinline__ mf_ef mf_ef_make(float v, float e) { mf_ef r; r.v = v; r.e = e; return r; }
+__device__ __forceinline__ mf_ef mf_ef_from(double x) {
+  const float v = (float)x;
+  return mf_ef_make(v, fabsf(v) * 0x1p-23f + 0x1p-126f);
+}
+__device__ __forceinline__ mf_ef mf_ef_neg(mf_ef a) { return mf_ef_make(-a.v, a.e); }
+__device__ __forceinline__ mf_ef mf_ef_add(mf_ef a, mf_ef b) {
+  const float v = a.v + b.v;
+  return mf_ef_make(v, fmaf(fabsf(v), 0x1p-23f, a.e + b.e));
+}
+__device__ __forceinline__ mf_ef mf_ef_sub(mf_ef a, mf_ef b) { return mf_ef_add(a, mf_ef_neg(b)); }
+__device__ __forceinline__ mf_ef mf_ef_mul(mf_ef a, mf_ef b) {
+  const float v = a.v * b.v;
+  return mf_ef_make(v, fmaf(fabsf(a.v) + a.e, b.e, fmaf(fabsf(b.v), a.e, fmaf(fabsf(v), 0x1p-23f, 0x1p-126f))));
+}
+__device__ __forceinline__ mf_ef mf_ef_rcp(mf_ef a) {  // |1/(a+d) - 1/a| <= e r^2 / (1 - e r)
+  const float r = __frcp_rn(a.v), er = a.e * fabsf(r);
+  return mf_ef_make(r, er < 0.25f ? fmaf(fabsf(r), fmaf(er, 1.34f, 0x1p-23f), 0x1p-126f) : MF_EF_INF);
+}
+// 4 units of 2^-23 of a function's result
+#define MF_EF_FN 0x1p-21f
+__device__ __forceinline__ mf_ef mf_ef_exp(mf_ef a) {  // e^d - 1 <= 1.07 d for d < 1/8
+  const float v = expf(a.v);
+  return mf_ef_make(v, a.e < 0.125f ? fmaf(v, fmaf(a.e, 1.07f, MF_EF_FN), 0x1p-126f) : MF_EF_INF);
+}
+__device__ __forceinline__ mf_ef mf_ef_log(mf_ef a) {
+  const float v = logf(a.v);
+  return mf_ef_make(v, a.v > 4.0f * a.e ? fmaf(fabsf(v), MF_EF_FN, 1.34f * a.e / a.v) : MF_EF_INF);
+}
+__device__ __forceinline__ mf_ef mf_ef_sqrt(mf_ef a) {  // |d| / (s + s') <= e / s
+  const float v = sqrtf(a.v);
+  return mf_ef_make(v, a.v > 2.0f * a.e ? fmaf(v, MF_EF_FN, 1.01f * a.e * rsqrtf(a.v)) : MF_EF_INF);
+}
+__device__ __forceinline__ void mf_ef_sincos(mf_ef a, mf_ef* s, mf_ef* c) {
+  sincosf(a.v, &s->v, &c->v);
+  s->e = fmaf(fabsf(s->v), MF_EF_FN, a.e) + 0x1p-126f;
+  c->e = fmaf(fabsf(c->v), MF_EF_FN, a.e) + 0x1p-126f;
+}
+__device__ __forceinline__ mf_ef mf_ef_sin(mf_ef a) {
+  const float v = sinf(a.v);
+  return mf_ef_make(v, fmaf(fabsf(v), MF_EF_FN, a.e) + 0x1p-126f);
+}
+__device__ __forceinline__ mf_ef mf_ef_cos(mf_ef a) {
+  const float v = cosf(a.v);
+  return mf_ef_make(v, fmaf(fabsf(v), MF_EF_FN, a.e) + 0x1p-126f);
+}
+__device__ __forceinline__ mf_ef mf_ef_tan(mf_ef a) {  // slope 1 + t^2, below 1.5 times that while e (1 + |t|) < 1/8
+  const float v = tanf(a.v);
+  return mf_ef_make(v, a.e * (1.0f + fabsf(v)) < 0.125f
+                           ? fmaf(fabsf(v), MF_EF_FN, a.e * fmaf(v, v, 1.0f) * 1.5f) + 0x1p-126f : MF_EF_INF);
+}
+__device__ __forceinline__ float mf_ef_arc(mf_ef a) {  // slope 1 / sqrt(1 - x^2) at the end of the interval nearest 1
+  const float y = (1.0f - fabsf(a.v)) - a.e;
+  return y > 1e-5f ? 1.01f * a.e * rsqrtf(y) : MF_EF_INF;
+}
+__device__ __forceinline__ mf_ef mf_ef_asin(mf_ef a) {
+  const float v = asinf(a.v);
+  return mf_ef_make(v, fmaf(fabsf(v), MF_EF_FN, mf_ef_arc(a)) + 0x1p-126f);
+}
+__device__ __forceinline__ mf_ef mf_ef_acos(mf_ef a) {
+  const float v = acosf(a.v);
+  return mf_ef_make(v, fmaf(fabsf(v), MF_EF_FN, mf_ef_arc(a)) + 0x1p-126f);
+}
+__device__ __forceinline__ mf_ef mf_ef_atan(mf_ef a) {
+  const float v = atanf(a.v);
+  return mf_ef_make(v, fmaf(fabsf(v), MF_EF_FN, a.e) + 0x1p-126f);
+}
+__device__ __forceinline__ mf_ef mf_ef_erf(mf_ef a) {
+  const float v = erff(a.v);
+  return mf_ef_make(v, fmaf(fabsf(v), MF_EF_FN, 1.13f * a.e) + 0x1p-126f);
+}
+// a^b for a > 0: ln of it moves by |b| de/a + |ln a| db; any other base in FP64
+__device__ __forceinline__ mf_ef mf_ef_pow(mf_ef a, mf_ef b) {
+  const float v = powf(a.v, b.v);
+  const float d = fmaf((fabsf(b.v) + b.e) * 1.34f, a.e / a.v, fabsf(logf(a.v)) * b.e * 1.01f);
+  return mf_ef_make(v, a.v > 4.0f * a.e && d < 0.125f ? fmaf(v, fmaf(d, 1.07f, 2.0f * MF_EF_FN), 0x1p-126f) : MF_EF_INF);
+}
+// whether the order of two values is uncertain
+__device__ __forceinline__ bool mf_ef_near(mf_ef a, mf_ef b) { return !(fabsf(a.v - b.v) > 1.01f * (a.e + b.e)); }
+)CUDA";
+
 // Bulk asynchronous global->shared copies completed on an mbarrier (sm_90+
 // PTX: cp.async.bulk, mbarrier.*). Both addresses 16-byte aligned, sizes a
 // multiple of 16 bytes.
@@ -1060,7 +1169,7 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
 
   LoweredKernel out;
   out.entry = "mf_" + std::string(kind == Kind::Reduce ? "reduce" : kind == Kind::Store ? "store" : "generate");
-  out.block = 256;
+  out.block = kind == Kind::Generate ? 128 : 256;
   out.vec = (kind == Kind::Generate) ? 1 : (st32 ? 4 : 2);
   if (kind == Kind::Reduce) {
     out.pipelined = !direct_loads;
@@ -1252,20 +1361,8 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
       if (n.op == Op::Param) return "p" + std::to_string(n.index);
       return "u" + std::to_string(k);
     };
-    // operands of which both sin and cos are live per-event values: node -> (sin node, cos node)
-    std::map<int, std::pair<int, int>> sincos_pair;
-    if (ar == Ar::DW) {
-      std::map<int, int> sin_of, cos_of;
-      for (size_t i = 0; i < ns.size(); i++) {
-        if (!live[i] || ns[i].uniform) continue;
-        if (ns[i].op == Op::Sin) sin_of[ns[i].a] = int(i);
-        if (ns[i].op == Op::Cos) cos_of[ns[i].a] = int(i);
-      }
-      for (auto& [a, si] : sin_of) {
-        auto c = cos_of.find(a);
-        if (c != cos_of.end()) sincos_pair[a] = {si, c->second};
-      }
-    }
+    std::map<int, std::pair<int, int>> sincos_pair;  // operand -> (sin node, cos node)
+    if (ar == Ar::DW) sincos_pair = sincos_pairs(ns, live);
     // Double-float REDUCE bodies: sums of (value x parameter-only factor)
     // terms become compensated dot products, and an output that is a product
     // used nowhere else is multiplied straight into its accumulator.
@@ -2204,36 +2301,31 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
     for (int j = 0; j < M; j++) s << "    outp[(mf_u64)" << j << " * out_stride + i] = (" << ST << ")r" << j << ";\n";
     s << "  }\n}\n";
   } else {
-    // GENERATE: one xoshiro128++ stream per thread, nper events per thread
-    // (thread t owns events [t*nper, min((t+1)*nper, n))).
+    // GENERATE: accept-reject generation, one xoshiro128++ stream per
+    // `lanes` threads of a warp (a power of two up to 32, chosen at launch).
+    // Stream t owns events [t*nper, min((t+1)*nper, n)) and makes them from
+    // its proposals in order. Lane j of the stream's lanes tests proposals j,
+    // lanes + j, ...: it starts (D+1) * j draws into the stream and skips the
+    // other lanes' (D+1) * (lanes - 1) draws after each of its own (six
+    // logic instructions a draw). The lanes' decisions meet in a ballot, and
+    // the accepted proposals take the stream's next events in the order of
+    // the proposals, so the events are those of one thread walking the
+    // stream, and no lane waits for another stream's next acceptance. Measured
+    // figures: generator_lanes() in mf_runtime.cpp.
     const int D = int(gen->dims.size());
     s << R"CUDA(__device__ __forceinline__ unsigned mf_rotl(unsigned x, int k) { return (x << k) | (x >> (32 - k)); }
-__device__ __forceinline__ unsigned mf_xoshiro(unsigned* s) {
-  const unsigned r = mf_rotl(s[0] + s[3], 7) + s[0];
-  const unsigned t = s[1] << 9;
-  s[2] ^= s[0]; s[3] ^= s[1]; s[1] ^= s[2]; s[0] ^= s[3]; s[2] ^= t; s[3] = mf_rotl(s[3], 11);
+struct mf_rng { unsigned s0, s1, s2, s3; };
+__device__ __forceinline__ void mf_rng_step(mf_rng& s) {
+  const unsigned t = s.s1 << 9, a = s.s2 ^ s.s0, b = s.s3 ^ s.s1;
+  s.s1 ^= a; s.s0 ^= b; s.s2 = a ^ t; s.s3 = mf_rotl(b, 11);
+}
+__device__ __forceinline__ unsigned mf_rng_draw(mf_rng& s) {
+  const unsigned r = mf_rotl(s.s0 + s.s3, 7) + s.s0;
+  mf_rng_step(s);
   return r;
 }
 )CUDA";
-    if (!ar32) s << dw_log_table() << kDwPrelude;
-    s << "extern \"C\" __global__ void __launch_bounds__(MF_BLOCK) " << out.entry
-      << "(const unsigned* __restrict__ seeds, unsigned nseeds, mf_u64 n, mf_u64 nper, mf_par P, " << ST
-      << "* __restrict__ outp, mf_u64 out_stride, unsigned* __restrict__ status, unsigned long long max_tries,"
-      << " unsigned long long splitmix_seed) {\n";
-    s << "  const unsigned t = blockIdx.x * MF_BLOCK + threadIdx.x;\n  if (t >= nseeds) return;\n";
-    // the stream's xoshiro128++ state: from the seed table, or (seeds null)
-    // made here as mf_splitmix_seed_rows makes row t: the upper halves of four
-    // SplitMix64 outputs (Steele, Lea and Flood, OOPSLA 2014) from
-    // (seed mod 2^32) * 2^32 + t
-    s << "  unsigned st[4];\n"
-      << "  if (seeds) {\n#pragma unroll\n    for (int k = 0; k < 4; k++) st[k] = seeds[(mf_u64)k * nseeds + t];\n"
-      << "  } else {\n    unsigned long long sm = (splitmix_seed & 0xffffffffull) * 4294967296ull + t;\n"
-      << "#pragma unroll\n    for (int k = 0; k < 4; k++) {\n"
-      << "      unsigned long long z = (sm += 0x9e3779b97f4a7c15ull);\n"
-      << "      z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;\n"
-      << "      z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;\n"
-      << "      st[k] = (unsigned)((z ^ (z >> 31)) >> 32);\n    }\n  }\n";
-    emit_params_and_uniform(s, "P.v");
+    if (!ar32) s << kEfPrelude;
     // The reference prints min, max-min and maxprob with "%.15e" into its
     // generate kernel (compute_llvm.hh:466-478,485-489) and evaluates
     // min + delta*u and maxprob*u with one rounding per operation; the
@@ -2246,154 +2338,225 @@ __device__ __forceinline__ unsigned mf_xoshiro(unsigned* s) {
     };
     const char* mul = ar32 ? "__fmul_rn" : "__dmul_rn";
     const char* add = ar32 ? "__fadd_rn" : "__dadd_rn";
-    // FP64 generation: the density is evaluated in double-float (FP32
-    // pairs on the FP32 pipe, which GB300 issues at 64x its FP64 rate:
-    // proposals split with integer operations, parameter-only values
-    // converted once per thread, tables from global memory), and the accept
-    // decision maxprob*u < p is recomputed with the density in exact FP64
-    // (the code the reference runs) whenever |maxprob*u - p| is within
-    // 1e-9 * maxprob or p is not finite. The double-float density is within
-    // about 1e-13 of the exact one when its intermediates stay inside the
-    // FP32 exponent range (2^-100 to 3.4e38 in magnitude, or zero), far
-    // inside that margin, so every decision -- and every generated event --
-    // equals the FP64 one. Only the proposals, the bound and the comparison
-    // stay on the FP64 pipe.
-    const bool fast_density = !ar32;
-    auto wref = [&](int id) -> std::string {
-      const Node& n = ns[id];
-      if (n.op == Op::Const) {
-        const float h = float(n.value);
-        const float l = float(n.value - double(h));
-        char b[96];
-        std::snprintf(b, sizeof b, "mf_dw_make(%af, %af)", double(h), double(l));
-        return b;
-      }
-      if (n.op == Op::Input) return "xw" + std::to_string(n.index);
-      if (n.op == Op::Param) return "pw" + std::to_string(n.index);
-      if (n.uniform) return "uw" + std::to_string(id);
-      return "w" + std::to_string(id);
+    // coordinate d from its draw (an expression), in the generated type; a
+    // draw times 2^-32 is exact in FP64 and one rounding of the draw in FP32
+    auto coordinate = [&](int d, const std::string& draw) {
+      return std::string(add) + "(" + fmt_const(printed15(gen->lo[d]), ar32) + ", " + mul + "(" +
+             fmt_const(printed15(gen->hi[d] - gen->lo[d]), ar32) + ", " +
+             (ar32 ? "(float)" + draw + " * 2.3283064365386963e-10f" : draw + " * 2.3283064365386963e-10") + "))";
     };
-    // sin and cos of one operand share a reduction: operand -> (sin node, cos node)
-    std::map<int, std::pair<int, int>> wsincos;
-    {
-      std::map<int, int> sin_of, cos_of;
-      for (size_t i = 0; i < ns.size(); i++) {
-        if (!live[i] || ns[i].uniform) continue;
-        if (ns[i].op == Op::Sin) sin_of[ns[i].a] = int(i);
-        if (ns[i].op == Op::Cos) cos_of[ns[i].a] = int(i);
-      }
-      for (auto& [a, si] : sin_of) {
-        auto c = cos_of.find(a);
-        if (c != cos_of.end()) wsincos[a] = {si, c->second};
-      }
-    }
-    auto wstmt = [&](int id) -> std::string {
-      const Node& n = ns[id];
-      const std::string lhs = "const " + std::string(n.op == Op::Cmp ? "bool" : "mf_dw") + " w" + std::to_string(id) + " = ";
-      const std::string A = n.a >= 0 ? wref(n.a) : "", B = n.b >= 0 ? wref(n.b) : "", Cc = n.c >= 0 ? wref(n.c) : "";
-      auto D = [](const std::string& v) { return "mf_dw_to_double(" + v + ")"; };
-      switch (n.op) {
-        case Op::Add: return lhs + "mf_dw_add(" + A + ", " + B + ");";
-        case Op::Sub: return lhs + "mf_dw_sub(" + A + ", " + B + ");";
-        case Op::Mul: return lhs + "mf_dw_mul(" + A + ", " + B + ");";
-        case Op::Div: return lhs + "mf_dw_mul(" + A + ", mf_dw_rcp(" + B + "));";
-        case Op::Neg: return lhs + "mf_dw_neg(" + A + ");";
-        case Op::Rcp: return lhs + "mf_dw_rcp(" + A + ");";
-        case Op::Log: return lhs + "mf_dw_log(" + A + ", mf_dw_logtab_g);";
-        case Op::Exp: return lhs + "mf_dw_exp(" + A + ", mf_dw_exptab_g);";
-        case Op::Pow: return lhs + "mf_dw_pow(" + A + ", " + B + ", mf_dw_logtab_g, mf_dw_exptab_g);";
-        case Op::Sqrt: return lhs + "mf_dw_sqrt(" + A + ");";
-        case Op::Sin:
-        case Op::Cos: {
-          auto it = wsincos.find(n.a);
-          if (it == wsincos.end()) return lhs + (n.op == Op::Sin ? "mf_dw_sin(" : "mf_dw_cos(") + A + ");";
-          if (id != std::min(it->second.first, it->second.second)) return "";  // defined with the first of the two
-          const std::string sn = "w" + std::to_string(it->second.first), cn = "w" + std::to_string(it->second.second);
-          return "mf_dw " + sn + ", " + cn + "; mf_dw_sincos(" + A + ", &" + sn + ", &" + cn + ");";
-        }
-        case Op::Cmp:
-          switch (n.cmp) {
-            case CmpOp::Gt: return lhs + "mf_dw_gt(" + A + ", " + B + ");";
-            case CmpOp::Lt: return lhs + "mf_dw_lt(" + A + ", " + B + ");";
-            case CmpOp::Ge: return lhs + "mf_dw_ge(" + A + ", " + B + ");";
-            case CmpOp::Le: return lhs + "mf_dw_le(" + A + ", " + B + ");";
-            case CmpOp::Eq: return lhs + "mf_dw_eq(" + A + ", " + B + ");";
-            case CmpOp::Ne: return lhs + "!mf_dw_eq(" + A + ", " + B + ");";
-          }
-          break;
-        case Op::Select: return lhs + "(" + A + " ? " + B + " : " + Cc + ");";
-        default:
-          if (is_unary_fn(n.op)) return lhs + "mf_dw_from_double(" + fn_name(n.op, false) + "(" + D(A) + "));";
-      }
-      throw std::runtime_error("emit: unexpected node");
-    };
-    // parameter-only values the double-float density reads, converted once per thread
-    auto emit_uniform_pairs = [&]() {
+    // FP64 generation decides maxprob*u < p in FP32 wherever that is certain:
+    // the density is evaluated in FP32 together with a bound of its error
+    // (kEfPrelude), and only where |maxprob*u - p| is within the bounds of
+    // both sides, or anything is not finite, are the coordinates and the
+    // density formed in FP64 (the code the reference runs) and compared. Every
+    // decision, and so every event, equals the FP64 one; GB300 issues FP64 at
+    // 1/64 of its FP32 rate. The accepted draws are stored in place of the
+    // coordinates and turned into coordinates, FP64 as the reference forms
+    // them, when the stream is complete (full warps instead of the few lanes
+    // that accept).
+    const bool filter = !ar32;
+    std::string filter_call;
+    std::vector<int> filter_uniform;
+    if (filter) {
       std::set<int> uni;
       auto note = [&](int k) {
         if (k >= 0 && ns[k].uniform && ns[k].op != Op::Const) uni.insert(k);
       };
+      std::set<int> conditions;  // parameter-only conditions of selects, exact
       for (size_t i = 0; i < ns.size(); i++) {
         if (!live[i] || ns[i].uniform || ns[i].op == Op::Input) continue;
-        note(ns[i].a);
+        const bool cond = ns[i].op == Op::Select && ns[ns[i].a].uniform;
+        if (cond) conditions.insert(ns[i].a);
+        if (!cond) note(ns[i].a);
         note(ns[i].b);
         note(ns[i].c);
       }
       for (int r : roots) note(r);
-      for (int k : uni) s << "  const mf_dw " << wref(k) << " = mf_dw_from_double(" << em.ref(k, "u") << ");\n";
-    };
-    auto accept_reject = [&]() {
-      if (fast_density) emit_uniform_pairs();
-      s << "  unsigned long long tries = 0;\n";
-      s << "  for (mf_u64 i = from; i < to; i++) {\n    for (;;) {\n";
-      s << "      if (++tries > max_tries) { atomicOr(status, 1u); return; }\n";
-      for (int d = 0; d < D; d++) {
-        s << "      const " << AT << " x" << d << " = " << add << "(" << fmt_const(printed15(gen->lo[d]), ar32) << ", "
-          << mul << "(" << fmt_const(printed15(gen->hi[d] - gen->lo[d]), ar32) << ", (" << AT
-          << ")(mf_xoshiro(st) * 2.3283064365386963e-10)));\n";
-      }
-      if (fast_density) {
-        for (int d = 0; d < D; d++) s << "      const mf_dw xw" << d << " = mf_dw_split_rn(x" << d << ");\n";
-        for (size_t i = 0; i < ns.size(); i++) {
-          if (!live[i] || ns[i].uniform || ns[i].op == Op::Input) continue;
-          const std::string st = wstmt(int(i));
-          if (!st.empty()) s << "      " << st << "\n";
+      auto eref = [&](int id) -> std::string {
+        const Node& n = ns[id];
+        if (n.op == Op::Const) {
+          const float v = float(n.value);
+          // the rounding of the constant, bounded (0 when it is exact)
+          const double e = std::isfinite(v) ? std::fabs(n.value - double(v)) * 1.0000005 : 0.0;
+          char b[96];
+          std::snprintf(b, sizeof b, "mf_ef_make(%s, %.9ef)", fmt_const(n.value, true).c_str(), e);
+          return b;
         }
-        s << "      const double mf_ug = " << mul << "(maxprob, (double)(mf_xoshiro(st) * 2.3283064365386963e-10));\n";
-        s << "      double mf_p = mf_dw_to_double_bits(" << wref(roots[0]) << ");\n";
-        s << "      if (!(fabs(mf_ug - mf_p) > 1e-9 * maxprob) || isinf(mf_p)) {  // exact FP64 density\n";
-        emit_body(s, "        ");
-        s << "        mf_p = r0;\n      }\n";
-        s << "      if (mf_ug < mf_p) {\n";
-      } else {
-        emit_body(s, "      ");
-        s << "      if (" << mul << "(maxprob, (" << AT << ")(mf_xoshiro(st) * 2.3283064365386963e-10)) < r0) {\n";
+        if (n.op == Op::Input) return "x" + std::to_string(n.index);
+        return (n.uniform ? "uf" : "f") + std::to_string(id);
+      };
+      s << "// The density in FP32 and a bound of its error; `amb` is set where a comparison is uncertain.\n"
+        << "__device__ __forceinline__ mf_ef mf_filter(";
+      for (int d = 0; d < D; d++) s << "mf_ef x" << d << ", ";
+      for (int k : uni) s << "mf_ef uf" << k << ", ";
+      for (int k : conditions) s << "bool uc" << k << ", ";
+      s << "bool& amb) {\n";
+      std::map<int, std::pair<int, int>> pair_of = sincos_pairs(ns, live);
+      for (size_t i = 0; i < ns.size(); i++) {
+        const Node& n = ns[i];
+        if (!live[i] || n.uniform || n.op == Op::Input) continue;
+        const std::string A = n.a >= 0 ? eref(n.a) : "", B = n.b >= 0 ? eref(n.b) : "", C = n.c >= 0 ? eref(n.c) : "";
+        const std::string lhs = "  const mf_ef f" + std::to_string(i) + " = ";
+        switch (n.op) {
+          case Op::Add: s << lhs << "mf_ef_add(" << A << ", " << B << ");\n"; break;
+          case Op::Sub: s << lhs << "mf_ef_sub(" << A << ", " << B << ");\n"; break;
+          case Op::Mul: s << lhs << "mf_ef_mul(" << A << ", " << B << ");\n"; break;
+          case Op::Div: s << lhs << "mf_ef_mul(" << A << ", mf_ef_rcp(" << B << "));\n"; break;
+          case Op::Neg: s << lhs << "mf_ef_neg(" << A << ");\n"; break;
+          case Op::Pow: s << lhs << "mf_ef_pow(" << A << ", " << B << ");\n"; break;
+          case Op::Cmp:
+            s << "  amb = amb || mf_ef_near(" << A << ", " << B << ");\n  const bool f" << i << " = " << A << ".v "
+              << cmp_str(n.cmp) << " " << B << ".v;\n";
+            break;
+          case Op::Select:
+            // a condition that is not a comparison tests a value against zero
+            if (ns[n.a].uniform)
+              s << lhs << "uc" << n.a << " ? " << B << " : " << C << ";\n";
+            else if (ns[n.a].op == Op::Cmp)
+              s << lhs << A << " ? " << B << " : " << C << ";\n";
+            else
+              s << "  amb = amb || mf_ef_near(" << A << ", mf_ef_make(0.0f, 0.0f));\n"
+                << lhs << A << ".v != 0.0f ? " << B << " : " << C << ";\n";
+            break;
+          case Op::Sin:
+          case Op::Cos: {
+            auto it = pair_of.find(n.a);
+            if (it == pair_of.end()) {
+              s << lhs << (n.op == Op::Sin ? "mf_ef_sin(" : "mf_ef_cos(") << A << ");\n";
+            } else if (int(i) == std::min(it->second.first, it->second.second)) {
+              s << "  mf_ef f" << it->second.first << ", f" << it->second.second << ";\n  mf_ef_sincos(" << A << ", &f"
+                << it->second.first << ", &f" << it->second.second << ");\n";
+            }
+            break;
+          }
+          default:
+            if (n.op != Op::Rcp && !is_unary_fn(n.op)) throw std::runtime_error("emit: unexpected node");
+            s << lhs << "mf_ef_" << (n.op == Op::Rcp ? "rcp" : fn_name(n.op, false)) << "(" << A << ");\n";
+        }
       }
-      for (int d = 0; d < D; d++)
-        s << "        outp[(mf_u64)" << d << " * out_stride + i] = (" << ST << ")x" << d << ";\n";
-      s << "        break;\n      }\n    }\n  }\n}\n";
+      s << "  return " << eref(roots[0]) << ";\n}\n";
+      filter_call = "mf_filter(";
+      for (int d = 0; d < D; d++) filter_call += "xe" + std::to_string(d) + ", ";
+      for (int k : uni) filter_call += "uf" + std::to_string(k) + ", ";
+      for (int k : conditions) filter_call += "(" + em.ref(k, "u") + ") != 0.0, ";
+      filter_call += "amb)";
+      for (int k : uni) filter_uniform.push_back(k);
+    }
+    // one stream's events, `lanes` threads a stream; from, to, maxprob and
+    // the parameter-only values are defined
+    auto accept_reject = [&]() {
+      for (int k : filter_uniform)
+        s << "  const mf_ef uf" << k << " = mf_ef_from(" << em.ref(k, "u") << ");\n";
+      if (filter) s << "  const mf_ef maxprob_f = mf_ef_from(maxprob);\n";
+      s << "  const unsigned sub = threadIdx.x & (lanes - 1u), first = (threadIdx.x & 31u) - sub;\n"
+        << "  const unsigned mine = lanes == 32u ? MF_FULL : ((1u << lanes) - 1u);\n"
+        << "  for (unsigned k = 0; k < sub; k++) {\n#pragma unroll\n    for (int q = 0; q < " << D + 1
+        << "; q++) mf_rng_step(st);\n  }\n"
+        << "  mf_u64 i = from, tried = 0;\n  bool run = i < to;\n"
+        << "  while (__any_sync(MF_FULL, run)) {\n";
+      for (int d = 0; d <= D; d++) s << "    const unsigned d" << d << " = mf_rng_draw(st);\n";
+      s << "    for (unsigned k = 1; k < lanes; k++) {\n#pragma unroll\n      for (int q = 0; q < " << D + 1
+        << "; q++) mf_rng_step(st);\n    }\n"
+        << "    bool acc = false;\n"
+        << "    if (run && tried + sub < max_tries) {\n";
+      auto draw = [](int d) { return "d" + std::to_string(d); };
+      if (filter) {
+        for (int d = 0; d < D; d++) {
+          const double lo = printed15(gen->lo[d]), del = printed15(gen->hi[d] - gen->lo[d]);
+          char eb[48];
+          std::snprintf(eb, sizeof eb, "%.9ef", (std::fabs(lo) + std::fabs(del)) * 0x1p-22);
+          s << "      const mf_ef xe" << d << " = mf_ef_make(__fmaf_rn(" << fmt_const(del, true) << ", (float)d" << d
+            << " * 2.3283064365386963e-10f, " << fmt_const(lo, true) << "), " << eb << ");\n";
+        }
+        s << "      bool amb = false;\n      const mf_ef p = " << filter_call << ";\n"
+          << "      const mf_ef ug = mf_ef_mul(maxprob_f, mf_ef_make((float)d" << D
+          << " * 2.3283064365386963e-10f, 0x1p-24f));\n"
+          << "      const float gap = __fsub_rn(p.v, ug.v);\n"
+          << "      acc = gap > 0.0f;\n"
+          << "      if (amb || !(fabsf(gap) > 1.01f * (p.e + ug.e) + 0x1p-23f * fabsf(gap))) {  // in FP64\n";
+        for (int d = 0; d < D; d++) s << "        const double x" << d << " = " << coordinate(d, draw(d)) << ";\n";
+        emit_body(s, "        ");
+        s << "        acc = __dmul_rn(maxprob, d" << D << " * 2.3283064365386963e-10) < r0;\n      }\n";
+      } else {
+        for (int d = 0; d < D; d++) s << "      const float x" << d << " = " << coordinate(d, draw(d)) << ";\n";
+        emit_body(s, "      ");
+        s << "      acc = __fmul_rn(maxprob, (float)d" << D << " * 2.3283064365386963e-10f) < r0;\n";
+      }
+      s << "    }\n"
+        << "    const unsigned m = (__ballot_sync(MF_FULL, acc) >> first) & mine;\n"
+        << "    if (acc) {\n      const mf_u64 at = i + __popc(m & ((1u << sub) - 1u));\n      if (at < to) {\n";
+      for (int d = 0; d < D; d++) {
+        const std::string slot = "outp[(mf_u64)" + std::to_string(d) + " * out_stride + at]";
+        if (filter)
+          s << "        " << slot << " = __longlong_as_double((long long)d" << d << ");\n";
+        else
+          s << "        " << slot << " = " << coordinate(d, draw(d)) << ";\n";
+      }
+      s << "      }\n    }\n"
+        << "    i += __popc(m);\n    tried += lanes;\n"
+        << "    if (run && i >= to) {\n      run = false;\n    } else if (run && tried >= max_tries) {\n"
+        << "      run = false;\n      if (sub == 0u) atomicOr(status, 1u);\n    }\n  }\n";
+      if (filter) {
+        s << "  // the stored draws become coordinates\n  __syncwarp();\n  if (i > to) i = to;\n"
+          << "  for (mf_u64 at = from + sub; at < i; at += lanes) {\n";
+        for (int d = 0; d < D; d++) {
+          const std::string slot = "outp[(mf_u64)" + std::to_string(d) + " * out_stride + at]";
+          s << "    { const unsigned w = (unsigned)__double_as_longlong(" << slot << ");\n      " << slot << " = "
+            << coordinate(d, "w") << "; }\n";
+        }
+        s << "  }\n";
+      }
+      s << "}\n";
     };
+    s << "extern \"C\" __global__ void __launch_bounds__(MF_BLOCK) " << out.entry
+      << "(const unsigned* __restrict__ seeds, unsigned nseeds, mf_u64 n, mf_u64 nper, mf_par P, " << ST
+      << "* __restrict__ outp, mf_u64 out_stride, unsigned* __restrict__ status, unsigned long long max_tries,"
+      << " unsigned long long splitmix_seed, unsigned lanes) {\n";
+    // whole warps stay in the loop: threads beyond the last stream have no events
+    s << "  const mf_u64 thread = (mf_u64)blockIdx.x * MF_BLOCK + threadIdx.x;\n"
+      << "  const bool have = thread / lanes < nseeds;\n"
+      << "  const unsigned t = have ? (unsigned)(thread / lanes) : 0u;\n";
+    // the stream's xoshiro128++ state: from the seed table, or (seeds null)
+    // made here as mf_splitmix_seed_rows makes row t: the upper halves of four
+    // SplitMix64 outputs (Steele, Lea and Flood, OOPSLA 2014) from
+    // (seed mod 2^32) * 2^32 + t
+    s << "  unsigned w[4];\n"
+      << "  if (seeds) {\n#pragma unroll\n    for (int k = 0; k < 4; k++) w[k] = seeds[(mf_u64)k * nseeds + t];\n"
+      << "  } else {\n    unsigned long long sm = (splitmix_seed & 0xffffffffull) * 4294967296ull + t;\n"
+      << "#pragma unroll\n    for (int k = 0; k < 4; k++) {\n"
+      << "      unsigned long long z = (sm += 0x9e3779b97f4a7c15ull);\n"
+      << "      z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;\n"
+      << "      z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;\n"
+      << "      w[k] = (unsigned)((z ^ (z >> 31)) >> 32);\n    }\n  }\n"
+      << "  mf_rng st = {w[0], w[1], w[2], w[3]};\n";
+    emit_params_and_uniform(s, "P.v");
     s << "  const " << AT << " maxprob = " << fmt_const(printed15(gen->maxprob), ar32) << ";\n";
-    s << "  const mf_u64 from = (mf_u64)t * nper;\n  mf_u64 to = from + nper; if (to > n) to = n;\n";
+    s << "  const mf_u64 from = have ? (mf_u64)t * nper : 0;\n"
+      << "  mf_u64 to = have ? from + nper : 0; if (to > n) to = n;\n";
     accept_reject();
     // Segments (toy studies): `threads_per_seg` streams per segment; segment
     // s owns events [seg_begin[s], seg_begin[s] + seg_count[s]) and generates
-    // them with its own parameter row and bound (thread r of the segment
+    // them with its own parameter row and bound (stream r of the segment
     // takes the r-th block of ceil(count / threads_per_seg) events).
     s << "extern \"C\" __global__ void __launch_bounds__(MF_BLOCK) " << out.entry
       << "_segments(const unsigned* __restrict__ seeds, unsigned nthreads, unsigned threads_per_seg,"
       << " const mf_u64* __restrict__ seg_begin, const unsigned* __restrict__ seg_count,"
       << " const mf_par* __restrict__ seg_params, const double* __restrict__ seg_maxprob, " << ST
-      << "* __restrict__ outp, mf_u64 out_stride, unsigned* __restrict__ status, unsigned long long max_tries) {\n";
-    s << "  const unsigned t = blockIdx.x * MF_BLOCK + threadIdx.x;\n  if (t >= nthreads) return;\n";
-    s << "  const unsigned seg = t / threads_per_seg, r = t - seg * threads_per_seg;\n";
-    s << "  unsigned st[4];\n#pragma unroll\n  for (int k = 0; k < 4; k++) st[k] = seeds[(mf_u64)k * nthreads + t];\n";
+      << "* __restrict__ outp, mf_u64 out_stride, unsigned* __restrict__ status, unsigned long long max_tries,"
+      << " unsigned lanes) {\n";
+    s << "  const mf_u64 thread = (mf_u64)blockIdx.x * MF_BLOCK + threadIdx.x;\n"
+      << "  const bool have = thread / lanes < nthreads;\n"
+      << "  const unsigned t = have ? (unsigned)(thread / lanes) : 0u;\n"
+      << "  const unsigned seg = t / threads_per_seg, r = t - seg * threads_per_seg;\n";
+    s << "  mf_rng st = {seeds[t], seeds[(mf_u64)nthreads + t], seeds[2 * (mf_u64)nthreads + t], "
+         "seeds[3 * (mf_u64)nthreads + t]};\n";
     s << "  const mf_par& P = seg_params[seg];\n";
     emit_params_and_uniform(s, "P.v");
     s << "  const " << AT << " maxprob = (" << AT << ")seg_maxprob[seg];\n";
-    s << "  const mf_u64 cnt = seg_count[seg], per = (cnt + threads_per_seg - 1) / threads_per_seg;\n";
-    s << "  const mf_u64 from = seg_begin[seg] + (mf_u64)r * per;\n";
-    s << "  mf_u64 to = from + per; if (to > seg_begin[seg] + cnt) to = seg_begin[seg] + cnt;\n";
+    s << "  const mf_u64 cnt = have ? seg_count[seg] : 0, per = (cnt + threads_per_seg - 1) / threads_per_seg;\n";
+    s << "  const mf_u64 end = seg_begin[seg] + cnt, from = seg_begin[seg] + (mf_u64)r * per;\n";
+    s << "  mf_u64 to = from + per; if (to > end) to = end;\n";
     accept_reject();
   }
   out.source = s.str();

@@ -2354,6 +2354,27 @@ int mf_kernel_store_async(mf_kernel* k, const mf_buffer* in, uint64_t in_stride,
   return kernel_store(k, in, in_stride, n, params, n_params, out, out_stride, false);
 }
 
+// Threads per stream of a GENERATE launch (see the generator in mf_lower.cpp):
+// enough that the streams fill the device with about 11 warps per SM, and at
+// least four. With one thread a stream a warp waits for the slowest of its 32
+// streams; every doubling halves that and the serial chain of a stream, and
+// costs one more pass of generator steps per proposal. FP64, one launch and
+// its wait on GB300 (before: one thread a stream, waiting for the warp's
+// slowest lane at every event, double-float density):
+//   threads per stream              1     4     8    16    32   before
+//   K*mumu P wave, 1M events      1127   379   337   373   532   4180 us
+//   S+P wave, 1M                   724   263   236   236   306
+//   mass, 1M                       239   106    96   103   148
+//   P wave, 50k (7143 streams)     153    69    56    58    72
+//   P wave, 1k (1000 streams)       68    37    31    29    28
+//   4096 toys, 65536 streams      3157  2757  2967  3559  4906 (with their tables)
+static unsigned generator_lanes(const mf_context* c, uint64_t streams) {
+  const uint64_t want = uint64_t(c->num_sms) * 352;
+  unsigned lanes = 4;
+  while (lanes < 32 && streams * lanes < want) lanes *= 2;
+  return lanes;
+}
+
 // seeds null: every stream seeded on the device from `splitmix_seed` (the
 // state mf_splitmix_seed_rows gives its row), no seed table copied.
 static int kernel_generate(mf_kernel* k, const uint32_t* seeds, uint32_t nseeds, uint64_t n, uint64_t nper,
@@ -2384,8 +2405,9 @@ static int kernel_generate(mf_kernel* k, const uint32_t* seeds, uint32_t nseeds,
   unsigned* status = c->status;
   unsigned long long mt = max_tries ? max_tries : 1000000000ULL;
   unsigned long long sms = splitmix_seed;
-  void* args[] = {&sd, &nseeds, &n, &nper, pv.data(), &outp, &out_stride, &status, &mt, &sms};
-  const unsigned grid = (nseeds + k->lowered.block - 1) / k->lowered.block;
+  unsigned lanes = generator_lanes(c, nseeds);
+  void* args[] = {&sd, &nseeds, &n, &nper, pv.data(), &outp, &out_stride, &status, &mt, &sms, &lanes};
+  const unsigned grid = unsigned((uint64_t(nseeds) * lanes + k->lowered.block - 1) / k->lowered.block);
   res_yield(k->ctx);
   MF_CUDA_TRY(cudaLaunchKernel(reinterpret_cast<const void*>(k->fn), dim3(grid), dim3(k->lowered.block), args, 0,
                                c->stream));
@@ -2460,9 +2482,10 @@ int mf_kernel_generate_segments(mf_kernel* k, const uint32_t* seeds, uint32_t nt
   void* outp = out->ptr;
   unsigned* status = c->status;
   unsigned long long mt = max_tries ? max_tries : 1000000000ULL;
+  unsigned lanes = generator_lanes(c, nthreads);
   void* args[] = {&d_seeds, &nthreads, &threads_per_seg, &d_begin, &d_count, const_cast<void**>(&d_par), &d_max,
-                  &outp, &out_stride, &status, &mt};
-  const unsigned grid = (nthreads + k->lowered.block - 1) / k->lowered.block;
+                  &outp, &out_stride, &status, &mt, &lanes};
+  const unsigned grid = unsigned((uint64_t(nthreads) * lanes + k->lowered.block - 1) / k->lowered.block);
   res_yield(k->ctx);
   MF_CUDA_TRY(cudaLaunchKernel(reinterpret_cast<const void*>(k->fn_seg), dim3(grid), dim3(k->lowered.block), args, 0,
                                c->stream));
