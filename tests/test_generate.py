@@ -104,6 +104,15 @@ extern "C" void run(int n, const float* xs, const float* e, const double* u, flo
     assert sure.mean() > 0.99 and np.median(q[sure]) < 1e-4 * maxprob
 
 
+@pytest.mark.parametrize("nrows,seed", [(1, 0), (2, 2**64 - 1), (257, 229387429), (8192, 12345)])
+def test_seed_rows_equal_the_stepped_jumps(nrows, seed):
+    """The table-driven jump gives the rows that stepping through the jump
+    polynomial gives (the C restatement)."""
+    from morefit_gb300.workloads import seed_rows
+    from oracle import mforacle
+    assert np.array_equal(seed_rows(nrows, seed), mforacle.seed_rows(nrows, seed))
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("workload", ["mass", "pwave"])
 @pytest.mark.parametrize("n", [1, 31, 1671, 1673, 6689, 8192, 8193, 100003])
