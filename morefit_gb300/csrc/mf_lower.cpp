@@ -902,6 +902,85 @@ __device__ __forceinline__ mf_dw mf_dw_shfl_xor(mf_dw a, int o) {
 }
 )CUDA";
 
+// Cross-thread sums of REDUCE kernels: double-float adds in a fixed order.
+// mf_sum_rows: the sums of `nb` partial rows, `step` rows apart, into sums[]
+// (shared, complete for every thread on return). Thread (g, o) takes rows g,
+// g + MF_GRP, ... of output o, so that a warp's loads are contiguous and a
+// round of loads covers MF_Q rows per thread, added as a tree; then MF_GRP
+// partials per output are added in order (few) or by a warp. Measured as part of a lone launch,
+// one thread per row and a shuffle tree per output took 18 us of the P-wave
+// Hessian's 54 (36 outputs, 152 rows, ncu) and 100 of the S+P wave's 163
+// (105 outputs, 608 rows).
+const char* kCombine = R"CUDA(
+template <int N> __device__ __forceinline__ void mf_warp_sums(mf_dw (&v)[N], int lane) {
+  int o = 16;
+#pragma unroll
+  for (int h = N / 2; h > 0; h >>= 1, o >>= 1) {
+    const bool up = (lane & o) != 0;  // keep the upper half of the outputs
+#pragma unroll
+    for (int c = 0; c < h; c++) {
+      const mf_dw keep = up ? v[c + h] : v[c], give = up ? v[c] : v[c + h];
+      v[c] = mf_dw_add(keep, mf_dw_shfl_xor(give, o));
+    }
+  }
+#pragma unroll
+  for (; o > 0; o >>= 1) v[0] = mf_dw_add(v[0], mf_dw_shfl_xor(v[0], o));
+}
+__device__ __forceinline__ void mf_sum_rows(const float2* rows, unsigned nb, unsigned step, float2* part, float2* sums) {
+  const mf_u64 stride = (mf_u64)step * MF_NOUT;
+#if MF_GRP > 1
+  const int g = threadIdx.x / MF_NOUT, o = threadIdx.x - g * MF_NOUT;
+  if (g < MF_GRP) {
+#else
+  const int g = 0;
+  for (int o = threadIdx.x; o < MF_NOUT; o += MF_BLOCK) {
+#endif
+    mf_dw a = mf_dw_make(0.0f, 0.0f);
+    for (unsigned r0 = g; r0 < nb; r0 += MF_GRP * MF_Q) {
+      float2 v[MF_Q];
+#pragma unroll
+      for (int q = 0; q < MF_Q; q++) {
+        const unsigned r = r0 + q * MF_GRP;
+        v[q] = r < nb ? __ldcg(rows + r * stride + o) : make_float2(0.0f, 0.0f);
+      }
+      mf_dw t[MF_Q];
+#pragma unroll
+      for (int q = 0; q < MF_Q; q++) t[q] = mf_dw_pair(v[q]);
+#pragma unroll
+      for (int h = MF_Q / 2; h > 0; h >>= 1)
+#pragma unroll
+        for (int q = 0; q < h; q++) t[q] = mf_dw_add(t[q], t[q + h]);
+      a = mf_dw_add(a, t[0]);
+    }
+#if MF_GRP > 1
+    part[g * MF_NOUT + o] = make_float2(a.h, a.l);
+  }
+  __syncthreads();
+#if MF_GRP <= 8
+  if (threadIdx.x < MF_NOUT) {
+    mf_dw a = mf_dw_pair(part[threadIdx.x]);
+#pragma unroll
+    for (int q = 1; q < MF_GRP; q++) a = mf_dw_add(a, mf_dw_pair(part[q * MF_NOUT + threadIdx.x]));
+    sums[threadIdx.x] = make_float2(a.h, a.l);
+  }
+#else
+  for (int j = threadIdx.x >> 5; j < MF_NOUT; j += MF_BLOCK / 32) {
+    mf_dw a = mf_dw_make(0.0f, 0.0f);
+#pragma unroll
+    for (int q = threadIdx.x & 31; q < MF_GRP; q += 32) a = mf_dw_add(a, mf_dw_pair(part[q * MF_NOUT + j]));
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) a = mf_dw_add(a, mf_dw_shfl_xor(a, w));
+    if ((threadIdx.x & 31) == 0) sums[j] = make_float2(a.h, a.l);
+  }
+#endif
+#else
+    sums[o] = make_float2(a.h, a.l);
+  }
+#endif
+  __syncthreads();
+}
+)CUDA";
+
 // FP32 values with a running bound of their error, for the generator's accept
 // test: the exact value of the expression lies within e of v. Every operation
 // adds to the propagated bounds of its operands the rounding of its own result
@@ -1256,18 +1335,16 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
   s << "#define MF_NREG " << NREG << "\n";
   // launch bounds of the event-loop entries
   s << "#define MF_BOUNDS __launch_bounds__(MF_BLOCK)\n";
-  // partial blocks each last-block thread loads per round (bounded register use)
-  // combine of block partial rows: MF_CC outputs at a time, MF_Q rows of each in flight per thread
-  // (up to 16 outputs and up to four rows of each, about 32 values per thread
-  // in flight: a grid of two blocks per SM leaves each thread of the last
-  // block one or two rows, so its loads go out in one round; many-output
-  // kernels, whose grids of small blocks leave thousands of partial rows, take
-  // eight outputs and four rows at a time)
-  const int cc = M > kAccRegMax ? 8 : std::min(M, 16);
-  s << "#define MF_CC " << cc << "\n";
-  s << "#define MF_Q " << (M > kAccRegMax ? 4 : std::max(1, std::min(4, 32 / cc))) << "\n";
-  // outputs per block-reduction chunk (one warp each)
-  s << "#define MF_RC " << std::max(1, std::min(8, out.block / 32)) << "\n";
+  // combine of block partial rows: MF_GRP threads share an output's rows, each
+  // with MF_Q loads in flight; kernels of many outputs, whose grids of small
+  // blocks leave hundreds of rows, combine them in groups of MF_ROWS blocks first
+  const int grp = std::max(1, out.block / M);
+  int q = 2;  // a power of two: the rows of a round are added as a tree
+  while (q < 16 && q * grp < 608) q *= 2;
+  s << "#define MF_GRP " << grp << "\n#define MF_Q " << q << "\n";
+  s << "#define MF_ROWS " << (M > kAccRegMax ? kCombineRows : 0) << "\n";
+  // shared scratch of the block reduction (a row per warp) and the combine (MF_GRP rows)
+  s << "#define MF_PART " << std::max(out.block / 32, grp) * M << "\n";
   s << "struct mf_par { double v[MF_NPAR]; };\n";
 
   // Parameter-only prologue (u*), emitted once per thread.
@@ -1925,40 +2002,59 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
         accs(ready_after[i]);
       }
     };
-    // A thread's partial of output J as a double-float value (expression).
-    auto thread_dw = [&](const std::string& J) -> std::string {
-      auto one = [&](const std::string& a, const std::string& c) {
-        if (ar == Ar::F32 || ar == Ar::F32S) return "mf_two_sum(" + a + ", -" + c + ")";
-        if (ar == Ar::F64) return "mf_dw_split(" + a + ")";
-        return "mf_dw_renorm(" + a + ")";
-      };
-      if (NREG == M) return one("acc[" + J + "]", "cmp[" + J + "]");
-      // J is a constant once the loop is unrolled; both indices stay in bounds
-      const std::string r = "((" + J + ") < MF_NREG ? (" + J + ") : 0)";
-      const std::string sh = "[(" + J + ") < MF_NREG ? 0 : (" + J + ") - MF_NREG][threadIdx.x]";
-      return "((" + J + ") < MF_NREG ? " + one("acc[" + r + "]", "cmp[" + r + "]") + " : " +
-             one("mf_sacc" + sh, "mf_scmp" + sh) + ")";
+    // A thread's partial of output j as a double-float value (expression).
+    auto thread_dw = [&](int j) -> std::string {
+      if (ar == Ar::F32 || ar == Ar::F32S) return "mf_two_sum(" + accref(j) + ", -" + cmpref(j) + ")";
+      if (ar == Ar::F64) return "mf_dw_split(" + accref(j) + ")";
+      return "mf_dw_renorm(" + accref(j) + ")";
     };
-    // Block reduction of every output into mf_blk[] (shared): outputs go in
-    // chunks of MF_RC through a [MF_RC][MF_BLOCK] staging array; warp w sums
-    // output j0 + w (each lane a fixed stride of threads, then a shuffle
-    // tree), so every output costs one warp's work instead of every warp's.
+    // Block reduction of every output into mf_blk[] (shared). A warp sums N
+    // outputs at once by a butterfly that halves the outputs a lane holds at
+    // every step (mf_warp_sums: N - 1 exchanges instead of 5 N), outputs going
+    // in chunks of 32, 16, 8, ... so that the fewest exchanges are made; then
+    // one thread per output adds the warps in order. One barrier, where
+    // staging eight outputs at a time through shared memory took two per
+    // chunk and one warp's serial sum each: the P-wave Hessian's 36 outputs
+    // were five such rounds, the S+P wave's 105 in blocks of two warps 53.
     // The order is fixed, so the result is reproducible.
+    const std::vector<int> chunks = [&] {
+      auto cost = [](int n) {  // exchanges of a chunk of n = 2^k outputs
+        int k = 0;
+        while ((1 << k) < n) k++;
+        return n - 1 + 5 - k;
+      };
+      std::vector<int> best(M + 1, 0), pick(M + 1, 0);
+      for (int r = 1; r <= M; r++)
+        for (int n = 1; n <= 32; n *= 2) {
+          const int c = cost(n) + best[std::max(0, r - n)];
+          if (!pick[r] || c < best[r]) {
+            best[r] = c;
+            pick[r] = n;
+          }
+        }
+      std::vector<int> v;
+      for (int r = M; r > 0; r -= pick[r]) v.push_back(pick[r]);
+      return v;
+    }();
     auto block_reduce = [&](std::ostringstream& o) {
-      o << "  __shared__ float2 mf_stage_red[MF_RC][MF_BLOCK];\n  __shared__ float2 mf_blk[MF_NOUT];\n"
-        << "  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;\n"
-        << "#pragma unroll\n  for (int j0 = 0; j0 < MF_NOUT; j0 += MF_RC) {\n"
-        << "#pragma unroll\n    for (int c = 0; c < MF_RC; c++)\n"
-        << "      if (j0 + c < MF_NOUT) {\n        const mf_dw t = " << thread_dw("j0 + c") << ";\n"
-        << "        mf_stage_red[c][threadIdx.x] = make_float2(t.h, t.l);\n      }\n"
-        << "    __syncthreads();\n"
-        << "    if (warp < MF_RC && j0 + warp < MF_NOUT) {\n"
-        << "      mf_dw a = mf_dw_make(mf_stage_red[warp][lane].x, mf_stage_red[warp][lane].y);\n"
-        << "#pragma unroll\n      for (int k = 1; k < MF_BLOCK / 32; k++)\n"
-        << "        a = mf_dw_add(a, mf_dw_make(mf_stage_red[warp][lane + 32 * k].x, mf_stage_red[warp][lane + 32 * k].y));\n"
-        << "#pragma unroll\n      for (int o = 16; o > 0; o >>= 1) a = mf_dw_add(a, mf_dw_shfl_xor(a, o));\n"
-        << "      if (lane == 0) mf_blk[j0 + warp] = make_float2(a.h, a.l);\n    }\n"
-        << "    __syncthreads();\n  }\n";
+      o << "  __shared__ float2 mf_part[MF_PART];\n  __shared__ float2 mf_blk[MF_NOUT];\n"
+        << "  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;\n";
+      int j0 = 0;
+      for (int n : chunks) {
+        o << "  {\n    mf_dw v[" << n << "];\n";
+        for (int c = 0; c < n; c++)
+          o << "    v[" << c << "] = " << (j0 + c < M ? thread_dw(j0 + c) : "mf_dw_make(0.0f, 0.0f)") << ";\n";
+        o << "    mf_warp_sums<" << n << ">(v, lane);\n"
+          << "    const int j = " << j0 << " + lane / " << 32 / n << ";\n"
+          << "    if (lane % " << 32 / n << " == 0 && j < MF_NOUT) mf_part[warp * MF_NOUT + j] = make_float2(v[0].h, v[0].l);\n"
+          << "  }\n";
+        j0 += n;
+      }
+      o << "  __syncthreads();\n"
+        << "  for (int j = threadIdx.x; j < MF_NOUT; j += MF_BLOCK) {\n"
+        << "    mf_dw a = mf_dw_pair(mf_part[j]);\n"
+        << "#pragma unroll\n    for (int w = 1; w < MF_BLOCK / 32; w++) a = mf_dw_add(a, mf_dw_pair(mf_part[w * MF_NOUT + j]));\n"
+        << "    mf_blk[j] = make_float2(a.h, a.l);\n  }\n  __syncthreads();\n";
     };
     bool f32_logprod = false;
     for (int j = 0; j < M; j++) f32_logprod = f32_logprod || (ar == Ar::F32 && logprod[j] >= 0);
@@ -1986,6 +2082,7 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
     const std::string XT = ar == Ar::F32 ? "float" : (ar == Ar::F64 || ar == Ar::F32S) ? "double" : "mf_dw";
 
     s << "struct mf_args { double d[" << out.nd << "]; float f[" << out.nf << "]; };\n";
+    s << kCombine;
     const auto entry_mark = s.tellp();
     // ---- single-dataset reduce ----
     s << "extern \"C\" __global__ void MF_BOUNDS " << out.entry << "(const " << DT
@@ -2083,70 +2180,43 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
       });
       s << "  }\n";
     }
-    s << "  __shared__ float2 red[MF_NOUT][MF_BLOCK / 32];\n  __shared__ bool am_last;\n";
+    s << "  __shared__ bool am_last;\n";
     acc_finish(s);
     block_reduce(s);
     // the per-block work, shared by the single-evaluation and the batched entry
     const std::string body_text = s.str().substr(size_t(body_mark));
-    // Fixed-order double-float combine of mf_nb partial rows (partials) into
-    // out[]: thread t takes rows t, t + MF_BLOCK, ... for every output (all
-    // loads of a round issued before the adds), then a warp tree and a pass
-    // over the warps in order. The order depends only on mf_nb, the grid size
-    // of the evaluation. Uses red[][], lane and warp.
-    // Outputs are combined MF_CC at a time (registers O(MF_CC), not
-    // O(MF_NOUT)); within each output the order is the one above, so the
-    // chunking changes no result.
-    const std::string combine_text = R"CUDA(  {
-    for (int j0 = 0; j0 < MF_NOUT; j0 += MF_CC) {
-      mf_dw s[MF_CC];
-#pragma unroll
-      for (int c = 0; c < MF_CC; c++) s[c] = mf_dw_make(0.0f, 0.0f);
-      for (unsigned b0 = 0; b0 < mf_nb; b0 += MF_Q * MF_BLOCK) {
-        float2 v[MF_Q][MF_CC];
-#pragma unroll
-        for (int q = 0; q < MF_Q; q++) {
-          const unsigned b = b0 + q * MF_BLOCK + threadIdx.x;
-#pragma unroll
-          for (int c = 0; c < MF_CC; c++)
-            v[q][c] = (b < mf_nb && j0 + c < MF_NOUT) ? __ldcg(partials + (mf_u64)b * MF_NOUT + j0 + c)
-                                                        : make_float2(0.0f, 0.0f);
-        }
-#pragma unroll
-        for (int q = 0; q < MF_Q; q++)
-#pragma unroll
-          for (int c = 0; c < MF_CC; c++) s[c] = mf_dw_add(s[c], mf_dw_make(v[q][c].x, v[q][c].y));
-      }
-#pragma unroll
-      for (int c = 0; c < MF_CC; c++) {
-        if (j0 + c >= MF_NOUT) break;
-        mf_dw a = s[c];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) a = mf_dw_add(a, mf_dw_shfl_xor(a, o));
-        if (lane == 0) red[j0 + c][warp] = make_float2(a.h, a.l);
-      }
-    }
-    __syncthreads();
-    for (int j = threadIdx.x; j < MF_NOUT; j += MF_BLOCK) {
-      mf_dw b = mf_dw_make(red[j][0].x, red[j][0].y);
-      for (int w = 1; w < MF_BLOCK / 32; w++) b = mf_dw_add(b, mf_dw_make(red[j][w].x, red[j][w].y));
-      out[j] = mf_dw_to_double(b);
-    }
-  }
-)CUDA";
     s << R"CUDA(  // Launched as a programmatic dependent of the previous evaluation on the
   // stream (batched evaluations), this grid ran its event loop while that
   // one finished; the scratch below is shared, so wait for it to complete.
   mf_grid_dependency_wait();
-  for (int j = threadIdx.x; j < MF_NOUT; j += MF_BLOCK) partials[(mf_u64)blockIdx.x * MF_NOUT + j] = mf_blk[j];
-  // Completion count with release/acquire semantics: the barrier orders the
-  // block's partial writes before thread 0's release; the last block's
-  // acquire plus the barrier orders its reads of every partial after.
-  __syncthreads();
-  if (threadIdx.x == 0) am_last = (mf_atom_add_acq_rel(counter, 1u) == gridDim.x - 1);
-  __syncthreads();
-  if (!am_last) return;
-  const unsigned mf_nb = gridDim.x;
-)CUDA" << combine_text << R"CUDA(  if (threadIdx.x == 0) *counter = 0u;
+  // Completion counts with release/acquire semantics: the barrier orders the
+  // block's row before thread 0's release; the last block's acquire plus the
+  // barrier orders its reads of every row after. A grid of one block has
+  // nothing to combine.
+  if (gridDim.x > 1u) {
+    for (int j = threadIdx.x; j < MF_NOUT; j += MF_BLOCK) partials[(mf_u64)blockIdx.x * MF_NOUT + j] = mf_blk[j];
+    __syncthreads();
+#if MF_ROWS > 0
+    const unsigned mf_g = blockIdx.x / MF_ROWS, mf_first = mf_g * MF_ROWS;
+    const unsigned mf_nr = gridDim.x - mf_first < MF_ROWS ? gridDim.x - mf_first : MF_ROWS;
+    if (threadIdx.x == 0) am_last = (mf_atom_add_acq_rel(counter + 1 + mf_g, 1u) == mf_nr - 1);
+    __syncthreads();
+    if (!am_last) return;
+    mf_sum_rows(partials + (mf_u64)mf_first * MF_NOUT, mf_nr, 1u, mf_part, mf_blk);
+    for (int j = threadIdx.x; j < MF_NOUT; j += MF_BLOCK) partials[(mf_u64)mf_first * MF_NOUT + j] = mf_blk[j];
+    if (threadIdx.x == 0) counter[1 + mf_g] = 0u;
+    __syncthreads();
+    const unsigned mf_nb = (gridDim.x + MF_ROWS - 1) / MF_ROWS, mf_step = MF_ROWS;
+#else
+    const unsigned mf_nb = gridDim.x, mf_step = 1u;
+#endif
+    if (threadIdx.x == 0) am_last = (mf_atom_add_acq_rel(counter, 1u) == mf_nb - 1);
+    __syncthreads();
+    if (!am_last) return;
+    mf_sum_rows(partials, mf_nb, mf_step, mf_part, mf_blk);
+    if (threadIdx.x == 0) *counter = 0u;
+  }
+  for (int j = threadIdx.x; j < MF_NOUT; j += MF_BLOCK) out[j] = mf_dw_to_double(mf_dw_pair(mf_blk[j]));
   // Synchronous evaluation (seq != 0): out[] is mapped host memory; publish
   // completion in the mapped word status[1] after every output is visible
   // system-wide, so the host can read the sums without a stream synchronize.
@@ -2189,7 +2259,7 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
       << "  mf_grid_dependency_wait();\n"
       << "}\n";
     s << "extern \"C\" __global__ void __launch_bounds__(MF_BLOCK) " << out.entry
-      << "_combine(const float2* __restrict__ partials_all, mf_u64 pstride, const unsigned* __restrict__ grids,"
+      << "_combine(float2* __restrict__ partials_all, mf_u64 pstride, const unsigned* __restrict__ grids,"
       << " double* __restrict__ out_all, unsigned count, unsigned grid_all) {\n"
       << "  // launched as a programmatic dependent of the last evaluation: its partials\n"
       << "  // (and every earlier one's) are complete and visible after this\n"
@@ -2197,11 +2267,26 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
       << "  const unsigned e = blockIdx.x;\n  if (e >= count) return;\n"
       << "  // every evaluation's grid size, or (grids null) the one they all share\n"
       << "  const unsigned mf_nb = grids ? grids[e] : grid_all;\n"
-      << "  const float2* __restrict__ partials = partials_all + (mf_u64)e * pstride;\n"
+      << "  float2* __restrict__ partials = partials_all + (mf_u64)e * pstride;\n"
       << "  double* __restrict__ out = out_all + (mf_u64)e * MF_NOUT;\n"
-      << "  __shared__ float2 red[MF_NOUT][MF_BLOCK / 32];\n"
-      << "  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;\n"
-      << combine_text << "}\n";
+      << R"CUDA(  __shared__ float2 mf_part[MF_PART];
+  __shared__ float2 mf_blk[MF_NOUT];
+  unsigned mf_rows = mf_nb, mf_step = 1u;
+#if MF_ROWS > 0
+  if (mf_nb > 1u) {  // the single-evaluation entry's groups first
+    for (unsigned f = 0; f < mf_nb; f += MF_ROWS) {
+      mf_sum_rows(partials + (mf_u64)f * MF_NOUT, mf_nb - f < MF_ROWS ? mf_nb - f : MF_ROWS, 1u, mf_part, mf_blk);
+      for (int j = threadIdx.x; j < MF_NOUT; j += MF_BLOCK) partials[(mf_u64)f * MF_NOUT + j] = mf_blk[j];
+      __syncthreads();
+    }
+    mf_rows = (mf_nb + MF_ROWS - 1) / MF_ROWS;
+    mf_step = MF_ROWS;
+  }
+#endif
+  mf_sum_rows(partials, mf_rows, mf_step, mf_part, mf_blk);
+  for (int j = threadIdx.x; j < MF_NOUT; j += MF_BLOCK) out[j] = mf_dw_to_double(mf_dw_pair(mf_blk[j]));
+}
+)CUDA";
 
     // ---- ragged segments: one block per segment ----
     s << "extern \"C\" __global__ void __launch_bounds__(MF_BLOCK) " << out.entry << "_segments(const " << DT

@@ -23,6 +23,10 @@
 
 namespace mf {
 
+// Blocks whose partial rows a REDUCE kernel of many outputs combines first
+// (one completion counter each, behind the grid's own).
+constexpr int kCombineRows = 16;
+
 enum class Op : uint8_t {
   Const, Input, Param, Add, Sub, Mul, Neg, Rcp, Div, Exp, Log, Sqrt, Sin, Cos, Tan, Asin, Acos, Atan, Erf,
   Pow, Cmp, Select

@@ -379,12 +379,18 @@ void ctx_free(mf_context* c, void* p, uint64_t bytes) {
   }
 }
 
+// Completion counters of REDUCE launches: the grid's and one per
+// mf::kCombineRows blocks (at most 32 blocks per SM).
+size_t counter_bytes(const mf_context* c) {
+  return (1 + (size_t(c->num_sms) * 32 + mf::kCombineRows - 1) / mf::kCombineRows) * sizeof(unsigned);
+}
+
 // Reads (and clears) the kernels' error word after the stream has drained.
 int check_status(mf_context* c) {
   const unsigned st = *c->status_host;
   if (!st) return MF_OK;
   *c->status_host = 0u;
-  cudaMemsetAsync(c->counter, 0, sizeof(unsigned), c->stream);  // a block that gave up may have left it set
+  cudaMemsetAsync(c->counter, 0, counter_bytes(c), c->stream);  // a block that gave up may have left them set
   cudaStreamSynchronize(c->stream);
   return fail(MF_ERR_TIMEOUT, "a kernel gave up waiting for its input tiles (status " + std::to_string(st) + ")");
 }
@@ -595,8 +601,8 @@ int mf_context_create(int device, uint64_t hbm_budget_bytes, mf_context** out) {
   c->budget = hbm_budget_bytes;
   c->cache_limit = hbm_budget_bytes ? hbm_budget_bytes / 4 : (uint64_t(8) << 30);
   MF_CUDA_TRY(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
-  MF_CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&c->counter), sizeof(unsigned)));
-  MF_CUDA_TRY(cudaMemset(c->counter, 0, sizeof(unsigned)));
+  MF_CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&c->counter), counter_bytes(c.get())));
+  MF_CUDA_TRY(cudaMemset(c->counter, 0, counter_bytes(c.get())));
   MF_CUDA_TRY(cudaHostAlloc(reinterpret_cast<void**>(&c->status_host), 64, cudaHostAllocMapped));
   MF_CUDA_TRY(cudaHostGetDevicePointer(reinterpret_cast<void**>(&c->status), c->status_host, 0));
   // all words: [1] is the completion word the first synchronous call waits
@@ -1489,13 +1495,13 @@ int launch_batched(mf_kernel* k, uint32_t count, const void* const* data, const 
     if (!one_grid)
       MF_CUDA_TRY(cudaMemcpyAsync(c->ring_grids, grids.data(), m * sizeof(unsigned), cudaMemcpyHostToDevice,
                                   c->stream));
-    const float2* ring = c->ring;
+    float2* ring = c->ring;
     uint64_t ps = pstride;
     const unsigned* g = one_grid ? nullptr : c->ring_grids;
     unsigned grid_all = grids[0];
     double* o = static_cast<double*>(out->ptr) + uint64_t(first) * k->n_outputs;
     uint32_t mm = m;
-    void* cargs[] = {const_cast<float2**>(&ring), &ps, const_cast<unsigned**>(&g), &o, &mm, &grid_all};
+    void* cargs[] = {&ring, &ps, const_cast<unsigned**>(&g), &o, &mm, &grid_all};
     // a programmatic dependent of the chunk's last evaluation (which completes
     // after every earlier one): the combine is resident before that grid ends
     // and waits for it in the kernel (unless the grid table copy sits between)
@@ -1941,7 +1947,7 @@ void res_build(mf_context* c, std::vector<mf_kernel*> members) {
       cudaHostGetDevicePointer(reinterpret_cast<void**>(&r.mail_dev), r.mail, 0) != cudaSuccess ||
       cudaMalloc(reinterpret_cast<void**>(&r.req), sizeof(ResReq)) != cudaSuccess ||
       cudaMalloc(reinterpret_cast<void**>(&r.go), sizeof(unsigned)) != cudaSuccess ||
-      cudaMalloc(reinterpret_cast<void**>(&r.counter), sizeof(unsigned)) != cudaSuccess ||
+      cudaMalloc(reinterpret_cast<void**>(&r.counter), counter_bytes(c)) != cudaSuccess ||
       cudaMalloc(reinterpret_cast<void**>(&r.partials), std::max<size_t>(part, 1) * sizeof(float2)) != cudaSuccess ||
       cudaStreamCreateWithFlags(&r.stream, cudaStreamNonBlocking) != cudaSuccess)
     return give_up("resident scratch allocation");
@@ -1988,7 +1994,7 @@ bool res_start(mf_context* c) {
   unsigned long long idle = c->res_idle_ns;
   void* args[] = {&mail, &req, &go, &partials, &counter, &status, &idle};
   if (cudaMemsetAsync(r.go, 0, sizeof(unsigned), r.stream) != cudaSuccess ||
-      cudaMemsetAsync(r.counter, 0, sizeof(unsigned), r.stream) != cudaSuccess ||
+      cudaMemsetAsync(r.counter, 0, counter_bytes(c), r.stream) != cudaSuccess ||
       cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(r.fn), args) != cudaSuccess) {
     cudaGetLastError();
     res_end(c);
@@ -2619,11 +2625,10 @@ int launch_multi(mf_context* c, mf_kernel* k0, const std::vector<MultiItem>& ite
   res_yield(k0->ctx);
   MF_CUDA_TRY(cudaLaunchKernel(reinterpret_cast<const void*>(k0->fn_multi), dim3(unsigned(nseg)),
                                dim3(k0->lowered.block), margs, 0, c->stream));
-  const float2* cring = ring;
   uint64_t pstride = pmax * k0->n_outputs;
   unsigned count = unsigned(items.size());
   unsigned grid_all = 0;  // unused: per-item counts in d_grids
-  void* cargs[] = {const_cast<float2**>(&cring), &pstride, const_cast<unsigned**>(&d_grids), &out, &count,
+  void* cargs[] = {&ring, &pstride, const_cast<unsigned**>(&d_grids), &out, &count,
                    &grid_all};
   MF_CUDA_TRY(cudaLaunchKernel(reinterpret_cast<const void*>(k0->fn_combine), dim3(count), dim3(k0->lowered.block),
                                cargs, 0, c->stream));
