@@ -2083,108 +2083,145 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
 
     s << "struct mf_args { double d[" << out.nd << "]; float f[" << out.nf << "]; };\n";
     s << kCombine;
+    const int NC = int(out.used_inputs.size());
+    const std::string VT = V == 1 ? DT : pair ? "float4" : st32 ? (V == 4 ? "float4" : "float2") : "double2";
+    // The per-block work of the single-evaluation and the batched entry: the
+    // event loop and the block reduction. `prefetch`: a thread's next events
+    // are loaded while it computes its present ones, the first before the
+    // tables (the same events in the same order, so the same sums).
+    auto block_work = [&](std::ostringstream& s, const bool prefetch) {
+      s << "  mf_launch_dependents();  // the next evaluation may start its event loop on SMs this grid frees\n";
+      auto load_at = [&](int k, const std::string& at) {
+        return "__ldg(reinterpret_cast<const " + VT + "*>(data + (mf_u64)" + std::to_string(k) + " * stride + " + at + "))";
+      };
+      if (prefetch) {
+        s << "  const mf_u64 step = (mf_u64)gridDim.x * MF_BLOCK * " << V << ";\n"
+          << "  mf_u64 base = ((mf_u64)blockIdx.x * MF_BLOCK + threadIdx.x) * " << V << ";\n";
+        for (int k : out.used_inputs)
+          s << "  " << VT << " c" << k << " = base < n ? " << load_at(k, "base") << " : " << VT << "();\n";
+      }
+      load_table(s);
+      prologue(s, "P.");
+      acc_decl(s);
+      const char* comp[4] = {"x", "y", "z", "w"};
+      // event v of the vector loaded into l<k>
+      auto lane_of = [&](int k, int v) -> std::string {
+        const std::string l = "l" + std::to_string(k);
+        if (pair) return V == 1 ? l : "make_float2(" + l + "." + comp[2 * v] + ", " + l + "." + comp[2 * v + 1] + ")";
+        return V == 1 ? l : l + "." + comp[v];
+      };
+      auto emit_events = [&](const std::string& ind, const std::string& idx0, const std::string& valid_base,
+                             const std::function<std::string(int)>& src) {
+        for (int k : out.used_inputs)
+          if (src) s << ind << "const " << VT << " l" << k << " = " << src(k) << ";\n";
+        for (int v = 0; v < V; v++) {
+          s << ind << "{\n";
+          for (int k : out.used_inputs)
+            s << ind << "  const " << XT << " x" << k << " = " << input_value(lane_of(k, v)) << ";\n";
+          body_acc(s, ind + "  ", valid_base + " + " + std::to_string(v) + " < n");
+          s << ind << "}\n";
+        }
+        (void)idx0;
+      };
+      if (out.pipelined && NC > 0) {
+        // Persistent blocks; tile t (events [t*MF_TILE, (t+1)*MF_TILE) of every
+        // column read by the body) goes to block t % gridDim.x. Thread 0 keeps
+        // MF_STAGES - 1 tiles in flight with bulk asynchronous copies into a
+        // ring of shared-memory stages; all threads wait on the stage's
+        // mbarrier (bounded), compute from shared memory and release the stage.
+        const size_t es = st32 ? 4 : 8;  // float pairs are 8 bytes too
+        out.smem_bytes = size_t(out.stages) * NC * out.tile * es;
+        s << "#define MF_TILE " << out.tile << "\n#define MF_STAGES " << out.stages << "\n#define MF_NC " << NC << "\n";
+        s << "  extern __shared__ __align__(128) unsigned char mf_dyn[];\n";
+        s << "  " << DT << "* __restrict__ stage = reinterpret_cast<" << DT << "*>(mf_dyn);\n";
+        s << "  __shared__ __align__(8) unsigned long long mf_bar[MF_STAGES];\n";
+        s << "  const mf_u64 ntiles = (n + MF_TILE - 1) / MF_TILE;\n";
+        s << "  if (threadIdx.x == 0) {\n    for (int q = 0; q < MF_STAGES; q++) mf_mbar_init(&mf_bar[q], 1u);\n"
+          << "    mf_fence_mbar_init();\n  }\n  __syncthreads();\n";
+        // issue lambda as a macro-like block
+        std::ostringstream issue;
+        issue << "{ const mf_u64 t0 = (TL) * (mf_u64)MF_TILE; mf_u64 cnt = stride - t0; if (cnt > MF_TILE) cnt = MF_TILE;\n"
+              << "          const unsigned bytes = (unsigned)(cnt * sizeof(" << DT << "));\n"
+              << "          mf_mbar_expect_tx(&mf_bar[SL], bytes * MF_NC);\n";
+        for (int ci = 0; ci < NC; ci++)
+          issue << "          mf_bulk_g2s(stage + ((mf_u64)(SL) * MF_NC + " << ci << ") * MF_TILE, data + (mf_u64)"
+                << out.used_inputs[ci] << " * stride + t0, bytes, &mf_bar[SL]);\n";
+        issue << "        }";
+        auto issue_code = [&](const std::string& tl, const std::string& sl) {
+          std::string c = issue.str();
+          for (size_t p; (p = c.find("(TL)")) != std::string::npos;) c.replace(p, 4, "(" + tl + ")");
+          for (size_t p; (p = c.find("SL")) != std::string::npos;) c.replace(p, 2, sl);
+          return c;
+        };
+        s << "  unsigned issued = 0;  // tiles issued by thread 0 (valid in thread 0)\n";
+        s << "  if (threadIdx.x == 0)\n    for (int q = 0; q < MF_STAGES - 1; q++) {\n"
+          << "      const mf_u64 tl = blockIdx.x + (mf_u64)q * gridDim.x;\n      if (tl < ntiles) {\n        "
+          << issue_code("tl", "q") << "\n        issued++;\n      }\n    }\n";
+        s << "  unsigned it = 0;\n  bool aborted = false;\n";
+        s << "  for (mf_u64 tile = blockIdx.x; tile < ntiles; tile += gridDim.x, it++) {\n";
+        s << "    const unsigned sl = it % MF_STAGES, par = (it / MF_STAGES) & 1u;\n";
+        s << "    if (threadIdx.x == 0) {\n      const mf_u64 nt = tile + (mf_u64)(MF_STAGES - 1) * gridDim.x;\n"
+          << "      if (nt < ntiles) {\n        const unsigned ns = (it + MF_STAGES - 1) % MF_STAGES;\n"
+          << "        mf_fence_proxy_async();\n        " << issue_code("nt", "ns") << "\n        issued++;\n      }\n    }\n";
+        s << "    const bool ok = mf_mbar_wait_bounded(&mf_bar[sl], par);\n";
+        s << "    if (__syncthreads_or(!ok)) { aborted = true; break; }\n";
+        s << "    const " << DT << "* __restrict__ sb = stage + (mf_u64)sl * MF_NC * MF_TILE;\n";
+        s << "    const mf_u64 tbase = tile * (mf_u64)MF_TILE;\n";
+        s << "    {\n      const int e0 = threadIdx.x * " << V << ";\n";
+        std::map<int, int> colpos;
+        for (int ci = 0; ci < NC; ci++) colpos[out.used_inputs[ci]] = ci;
+        emit_events("      ", "e0", "tbase + e0", [&](int k) {
+          return "*reinterpret_cast<const " + VT + "*>(sb + " + std::to_string(colpos[k]) + " * MF_TILE + e0)";
+        });
+        s << "    }\n    __syncthreads();\n  }\n";
+        // abort: report, drain this block's copies still in flight (bounded), continue to the reduction
+        s << "  if (aborted && threadIdx.x == 0) {\n    atomicOr(status, 1u);\n"
+          << "    for (unsigned k = it; k < issued; k++) mf_mbar_wait_bounded(&mf_bar[k % MF_STAGES], (k / MF_STAGES) & 1u);\n"
+          << "  }\n";
+      } else if (prefetch) {
+        if (out.stages > 1) s << "#pragma unroll " << out.stages << "\n";
+        s << "  for (; base < n; base += step) {\n    const mf_u64 ahead = base + step;\n";
+        for (int k : out.used_inputs) s << "    const " << VT << " l" << k << " = c" << k << ";\n";
+        for (int k : out.used_inputs)
+          s << "    c" << k << " = ahead < n ? " << load_at(k, "ahead") << " : " << VT << "();\n";
+        emit_events("    ", "base", "base", nullptr);
+        s << "  }\n";
+      } else {
+        s << "  const mf_u64 step = (mf_u64)gridDim.x * MF_BLOCK * " << V << ";\n";
+        // unrolled: the next iteration's loads are issued before this one's arithmetic
+        if (out.stages > 1) s << "#pragma unroll " << out.stages << "\n";
+        s << "  for (mf_u64 base = ((mf_u64)blockIdx.x * MF_BLOCK + threadIdx.x) * " << V
+          << "; base < n; base += step) {\n";
+        emit_events("    ", "base", "base", [&](int k) { return load_at(k, "base"); });
+        s << "  }\n";
+      }
+      s << "  __shared__ bool am_last;\n";
+      acc_finish(s);
+      block_reduce(s);
+    };
+    // Prefetching pays where one launch must hide its own latency (a lone
+    // evaluation: the P-wave Hessian's eight warps per SM keep 18 KB of loads
+    // in flight without it, which is 2.8 TB/s) and the next events fit in
+    // registers beside the accumulators at the same blocks per SM. Lone calls,
+    // 1M events (S+P FP32: 3M), without and with: P wave gradient 30.4 / 27.3
+    // us, value 26.5 / 25.9, Hessian 54.8 / 45.5, S+P gradient 52.6 / 45.6,
+    // value 33.8 / 32.4, P wave FP32 gradient 21.5 / 20.2, mass FP32 22.4 /
+    // 21.5; but P wave FP32 Hessian 30.9 / 34.2 and S+P FP32 gradient 44.4 /
+    // 50.1 (a block per SM fewer), and the S+P Hessian spills. Batched
+    // evaluations overlap their neighbours instead and keep the registers
+    // (P-wave gradient, 64 points of 100k events: 175 without, 190 with).
+    const bool lone_prefetch = !out.pipelined && NC > 0 &&
+                               (ar == Ar::DW ? M <= kAccRegMax : ar != Ar::F64 && M <= 16 && NC * V <= 40);
+    std::ostringstream lone_work, part_work;
+    block_work(lone_work, lone_prefetch);
+    block_work(part_work, false);
     const auto entry_mark = s.tellp();
     // ---- single-dataset reduce ----
     s << "extern \"C\" __global__ void MF_BOUNDS " << out.entry << "(const " << DT
       << "* __restrict__ data, mf_u64 stride, mf_u64 n, mf_args P, float2* __restrict__ partials,"
       << " unsigned* __restrict__ counter, double* __restrict__ out, unsigned* __restrict__ status, unsigned seq) {\n";
     const auto body_mark = s.tellp();
-    s << "  mf_launch_dependents();  // the next evaluation may start its event loop on SMs this grid frees\n";
-    load_table(s);
-    prologue(s, "P.");
-    acc_decl(s);
-    const std::string VT = V == 1 ? DT : pair ? "float4" : st32 ? (V == 4 ? "float4" : "float2") : "double2";
-    const char* comp[4] = {"x", "y", "z", "w"};
-    // event v of the vector loaded into l<k>
-    auto lane_of = [&](int k, int v) -> std::string {
-      const std::string l = "l" + std::to_string(k);
-      if (pair) return V == 1 ? l : "make_float2(" + l + "." + comp[2 * v] + ", " + l + "." + comp[2 * v + 1] + ")";
-      return V == 1 ? l : l + "." + comp[v];
-    };
-    auto emit_events = [&](const std::string& ind, const std::string& idx0, const std::string& valid_base,
-                           const std::function<std::string(int)>& src) {
-      for (int k : out.used_inputs) s << ind << "const " << VT << " l" << k << " = " << src(k) << ";\n";
-      for (int v = 0; v < V; v++) {
-        s << ind << "{\n";
-        for (int k : out.used_inputs)
-          s << ind << "  const " << XT << " x" << k << " = " << input_value(lane_of(k, v)) << ";\n";
-        body_acc(s, ind + "  ", valid_base + " + " + std::to_string(v) + " < n");
-        s << ind << "}\n";
-      }
-      (void)idx0;
-    };
-    const int NC = int(out.used_inputs.size());
-    if (out.pipelined && NC > 0) {
-      // Persistent blocks; tile t (events [t*MF_TILE, (t+1)*MF_TILE) of every
-      // column read by the body) goes to block t % gridDim.x. Thread 0 keeps
-      // MF_STAGES - 1 tiles in flight with bulk asynchronous copies into a
-      // ring of shared-memory stages; all threads wait on the stage's
-      // mbarrier (bounded), compute from shared memory and release the stage.
-      const size_t es = st32 ? 4 : 8;  // float pairs are 8 bytes too
-      out.smem_bytes = size_t(out.stages) * NC * out.tile * es;
-      s << "#define MF_TILE " << out.tile << "\n#define MF_STAGES " << out.stages << "\n#define MF_NC " << NC << "\n";
-      s << "  extern __shared__ __align__(128) unsigned char mf_dyn[];\n";
-      s << "  " << DT << "* __restrict__ stage = reinterpret_cast<" << DT << "*>(mf_dyn);\n";
-      s << "  __shared__ __align__(8) unsigned long long mf_bar[MF_STAGES];\n";
-      s << "  const mf_u64 ntiles = (n + MF_TILE - 1) / MF_TILE;\n";
-      s << "  if (threadIdx.x == 0) {\n    for (int q = 0; q < MF_STAGES; q++) mf_mbar_init(&mf_bar[q], 1u);\n"
-        << "    mf_fence_mbar_init();\n  }\n  __syncthreads();\n";
-      // issue lambda as a macro-like block
-      std::ostringstream issue;
-      issue << "{ const mf_u64 t0 = (TL) * (mf_u64)MF_TILE; mf_u64 cnt = stride - t0; if (cnt > MF_TILE) cnt = MF_TILE;\n"
-            << "          const unsigned bytes = (unsigned)(cnt * sizeof(" << DT << "));\n"
-            << "          mf_mbar_expect_tx(&mf_bar[SL], bytes * MF_NC);\n";
-      for (int ci = 0; ci < NC; ci++)
-        issue << "          mf_bulk_g2s(stage + ((mf_u64)(SL) * MF_NC + " << ci << ") * MF_TILE, data + (mf_u64)"
-              << out.used_inputs[ci] << " * stride + t0, bytes, &mf_bar[SL]);\n";
-      issue << "        }";
-      auto issue_code = [&](const std::string& tl, const std::string& sl) {
-        std::string c = issue.str();
-        for (size_t p; (p = c.find("(TL)")) != std::string::npos;) c.replace(p, 4, "(" + tl + ")");
-        for (size_t p; (p = c.find("SL")) != std::string::npos;) c.replace(p, 2, sl);
-        return c;
-      };
-      s << "  unsigned issued = 0;  // tiles issued by thread 0 (valid in thread 0)\n";
-      s << "  if (threadIdx.x == 0)\n    for (int q = 0; q < MF_STAGES - 1; q++) {\n"
-        << "      const mf_u64 tl = blockIdx.x + (mf_u64)q * gridDim.x;\n      if (tl < ntiles) {\n        "
-        << issue_code("tl", "q") << "\n        issued++;\n      }\n    }\n";
-      s << "  unsigned it = 0;\n  bool aborted = false;\n";
-      s << "  for (mf_u64 tile = blockIdx.x; tile < ntiles; tile += gridDim.x, it++) {\n";
-      s << "    const unsigned sl = it % MF_STAGES, par = (it / MF_STAGES) & 1u;\n";
-      s << "    if (threadIdx.x == 0) {\n      const mf_u64 nt = tile + (mf_u64)(MF_STAGES - 1) * gridDim.x;\n"
-        << "      if (nt < ntiles) {\n        const unsigned ns = (it + MF_STAGES - 1) % MF_STAGES;\n"
-        << "        mf_fence_proxy_async();\n        " << issue_code("nt", "ns") << "\n        issued++;\n      }\n    }\n";
-      s << "    const bool ok = mf_mbar_wait_bounded(&mf_bar[sl], par);\n";
-      s << "    if (__syncthreads_or(!ok)) { aborted = true; break; }\n";
-      s << "    const " << DT << "* __restrict__ sb = stage + (mf_u64)sl * MF_NC * MF_TILE;\n";
-      s << "    const mf_u64 tbase = tile * (mf_u64)MF_TILE;\n";
-      s << "    {\n      const int e0 = threadIdx.x * " << V << ";\n";
-      std::map<int, int> colpos;
-      for (int ci = 0; ci < NC; ci++) colpos[out.used_inputs[ci]] = ci;
-      emit_events("      ", "e0", "tbase + e0", [&](int k) {
-        return "*reinterpret_cast<const " + VT + "*>(sb + " + std::to_string(colpos[k]) + " * MF_TILE + e0)";
-      });
-      s << "    }\n    __syncthreads();\n  }\n";
-      // abort: report, drain this block's copies still in flight (bounded), continue to the reduction
-      s << "  if (aborted && threadIdx.x == 0) {\n    atomicOr(status, 1u);\n"
-        << "    for (unsigned k = it; k < issued; k++) mf_mbar_wait_bounded(&mf_bar[k % MF_STAGES], (k / MF_STAGES) & 1u);\n"
-        << "  }\n";
-    } else {
-      s << "  const mf_u64 step = (mf_u64)gridDim.x * MF_BLOCK * " << V << ";\n";
-      // unrolled: the next iteration's loads are issued before this one's arithmetic
-      if (out.stages > 1) s << "#pragma unroll " << out.stages << "\n";
-      s << "  for (mf_u64 base = ((mf_u64)blockIdx.x * MF_BLOCK + threadIdx.x) * " << V
-        << "; base < n; base += step) {\n";
-      emit_events("    ", "base", "base", [&](int k) {
-        return "__ldg(reinterpret_cast<const " + VT + "*>(data + (mf_u64)" + std::to_string(k) + " * stride + base))";
-      });
-      s << "  }\n";
-    }
-    s << "  __shared__ bool am_last;\n";
-    acc_finish(s);
-    block_reduce(s);
-    // the per-block work, shared by the single-evaluation and the batched entry
-    const std::string body_text = s.str().substr(size_t(body_mark));
+    s << lone_work.str();
     s << R"CUDA(  // Launched as a programmatic dependent of the previous evaluation on the
   // stream (batched evaluations), this grid ran its event loop while that
   // one finished; the scratch below is shared, so wait for it to complete.
@@ -2227,19 +2264,23 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
   }
 )CUDA";
     if (!out.pipelined) {
-      std::string work = s.str().substr(size_t(body_mark));
-      auto replace_all = [](std::string& t, const std::string& from, const std::string& to) {
-        for (size_t p = t.find(from); p != std::string::npos; p = t.find(from, p + to.size())) t.replace(p, from.size(), to);
+      const std::string tail = s.str().substr(size_t(body_mark) + lone_work.str().size());
+      auto resident = [&](std::string work) {
+        auto replace_all = [](std::string& t, const std::string& from, const std::string& to) {
+          for (size_t p = t.find(from); p != std::string::npos; p = t.find(from, p + to.size())) t.replace(p, from.size(), to);
+        };
+        replace_all(work, "blockIdx.x", "mf_vb");
+        replace_all(work, "gridDim.x", "mf_grid");
+        return "__device__ __forceinline__ void mf_rbody(const " + DT +
+               "* __restrict__ data, mf_u64 stride, mf_u64 n, const mf_args& P, float2* __restrict__ "
+               "partials, unsigned* __restrict__ counter, double* __restrict__ out, unsigned* "
+               "__restrict__ status, unsigned seq, unsigned mf_vb, unsigned mf_grid) {\n" +
+               work + "}\n";
       };
-      replace_all(work, "blockIdx.x", "mf_vb");
-      replace_all(work, "gridDim.x", "mf_grid");
       out.resident_prefix = s.str().substr(0, size_t(entry_mark));
       out.resident_data_type = DT;
-      out.resident_body = "__device__ __forceinline__ void mf_rbody(const " + DT +
-                          "* __restrict__ data, mf_u64 stride, mf_u64 n, const mf_args& P, float2* __restrict__ "
-                          "partials, unsigned* __restrict__ counter, double* __restrict__ out, unsigned* "
-                          "__restrict__ status, unsigned seq, unsigned mf_vb, unsigned mf_grid) {\n" +
-                          work + "}\n";
+      out.resident_body = resident(lone_work.str() + tail);
+      out.resident_plain = resident(part_work.str() + tail);
     }
     s << "}\n";
     // ---- batched evaluations: per-block partials only, then one combine ----
@@ -2252,7 +2293,7 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
     s << "extern \"C\" __global__ void MF_BOUNDS " << out.entry << "_part(const " << DT
       << "* __restrict__ data, mf_u64 stride, mf_u64 n, mf_args P, float2* __restrict__ partials,"
       << " unsigned* __restrict__ status) {\n"
-      << body_text
+      << part_work.str()
       << "  for (int j = threadIdx.x; j < MF_NOUT; j += MF_BLOCK) partials[(mf_u64)blockIdx.x * MF_NOUT + j] = mf_blk[j];\n"
       << "  // complete only after the previous evaluation's grid: completions stay in\n"
       << "  // stream order, so the combine launch after the last evaluation sees every partial\n"

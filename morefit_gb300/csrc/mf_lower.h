@@ -102,7 +102,8 @@ struct LoweredKernel {
   //            status, seq, unsigned block, unsigned grid)
   // doing block `block` of a grid of `grid` blocks, i.e. the entry with
   // blockIdx.x and gridDim.x replaced. Empty when not available.
-  std::string resident_prefix, resident_body;
+  // resident_plain is the same without prefetching, in fewer registers.
+  std::string resident_prefix, resident_body, resident_plain;
   std::string resident_data_type;  // element type mf_rbody reads ("float2", "double", "float")
   size_t smem_bytes = 0;  // dynamic shared memory of the main entry
   // REDUCE kernels: host-evaluated argument struct

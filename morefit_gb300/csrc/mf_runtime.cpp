@@ -1771,12 +1771,13 @@ void res_forget(mf_kernel* k) {
 // The resident module's source: every member's translation unit up to its
 // entry points plus mf_rbody, in namespace mfr<i> (its macros undefined after
 // it), and the resident entry.
-std::string res_source(const std::vector<const mf::LoweredKernel*>& m, int block, int min_blocks = 1) {
+std::string res_source(const std::vector<const mf::LoweredKernel*>& m, int block, int min_blocks, bool plain) {
   std::ostringstream s;
   s << "// MoreFit CUDA backend: resident evaluations of " << m.size() << " REDUCE kernels\n";
   for (size_t i = 0; i < m.size(); i++) {
     const mf::LoweredKernel& L = *m[i];
-    s << "namespace mfr" << i << " {\n" << L.resident_prefix << L.resident_body << "}  // namespace mfr" << i << "\n";
+    s << "namespace mfr" << i << " {\n" << L.resident_prefix << (plain ? L.resident_plain : L.resident_body)
+      << "}  // namespace mfr" << i << "\n";
     std::vector<std::string> macros;
     std::istringstream t(L.resident_prefix);
     for (std::string line; std::getline(t, line);)
@@ -1926,12 +1927,14 @@ void res_build(mf_context* c, std::vector<mf_kernel*> members) {
   }
   // as many resident blocks per SM as the member that launches the most
   // (fewer make its blocks run in rounds): the largest count down from there
-  // whose register cap spills no more than the kernels themselves
+  // whose register cap spills no more than the kernels themselves, with the
+  // prefetching event loops where those fit
   std::shared_ptr<CompiledImage> img;
   for (int mb = want; mb >= 1 && !img; mb--)
-    if (compile_source(res_source(lowered, block, mb), "mf_resident", img, "mf_resident") != MF_OK ||
-        img->spill > member_spill)
-      img.reset();
+    for (int plain = 0; plain < 2 && !img; plain++)
+      if (compile_source(res_source(lowered, block, mb, plain != 0), "mf_resident", img, "mf_resident") != MF_OK ||
+          img->spill > member_spill)
+        img.reset();
   if (!img) return give_up("the resident module spills more than its kernels");
   if (cudaLibraryLoadData(&r.lib, img->cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0) != cudaSuccess ||
       cudaLibraryGetKernel(&r.fn, r.lib, "mf_resident") != cudaSuccess)
@@ -2140,15 +2143,19 @@ int mf_compile_check_resident(const mf_kernel_desc* const* descs, uint32_t count
     if (lk[i].block != lk[0].block) return fail(MF_ERR_INVALID, "members differ in block size");
     ptrs.push_back(&lk[i]);
   }
-  const std::string src = res_source(ptrs, lk[0].block);
+  std::string src;
+  std::shared_ptr<CompiledImage> img;
+  for (int plain = 0; plain < 2; plain++) {
+    src = res_source(ptrs, lk[0].block, 1, plain != 0);
+    int rc = compile_source(src, "mf_resident", img, "mf_resident");
+    if (rc) return rc;
+    if (img->spill == 0) break;
+  }
   if (source && len) {
     const size_t n = std::min(len - 1, src.size());
     std::memcpy(source, src.data(), n);
     source[n] = '\0';
   }
-  std::shared_ptr<CompiledImage> img;
-  int rc = compile_source(src, "mf_resident", img, "mf_resident");
-  if (rc) return rc;
   if (regs) *regs = img->regs;
   if (spill) *spill = img->spill;
   return MF_OK;
