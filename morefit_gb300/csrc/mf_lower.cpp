@@ -2329,25 +2329,49 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
 }
 )CUDA";
 
+    // Event loop and block reduction of a block that owns events [first,
+    // first + cnt) of its columns, its parameters in `P`: one event per thread
+    // and round, the next round's event loaded while this one is computed (the
+    // first before the tables): a block is alone with its segment and its few
+    // warps hide little latency. Toys of 2000 P-wave events, one call, plain
+    // and so: value of 1 toy 52 / 37 us, of 1000 144 / 112, of 4096 388 / 315;
+    // F, gradient and Hessian of 1000 toys 311 / 304. Kernels whose partials
+    // fill the registers (more than kAccRegMax outputs) keep the plain loop.
+    const bool seg_prefetch = M <= kAccRegMax;
+    auto segment_work = [&](std::ostringstream& o) {
+      auto load_event = [&](int k, const std::string& at) {
+        return "__ldg(data + (mf_u64)" + std::to_string(k) + " * stride + first + " + at + ")";
+      };
+      if (seg_prefetch)
+        for (int k : out.used_inputs)
+          o << "  " << DT << " c" << k << " = threadIdx.x < cnt ? " << load_event(k, "threadIdx.x") << " : " << DT
+            << "();\n";
+      load_table(o);
+      prologue(o, "P.");
+      acc_decl(o);
+      o << "  for (unsigned i = threadIdx.x; i < cnt; i += MF_BLOCK) {\n";
+      if (seg_prefetch) {
+        for (int k : out.used_inputs) o << "    const " << DT << " l" << k << " = c" << k << ";\n";
+        o << "    const unsigned ahead = i + MF_BLOCK;\n";
+        for (int k : out.used_inputs)
+          o << "    c" << k << " = ahead < cnt ? " << load_event(k, "ahead") << " : " << DT << "();\n";
+      }
+      for (int k : out.used_inputs)
+        o << "    const " << XT << " x" << k << " = "
+          << input_value(seg_prefetch ? "l" + std::to_string(k) : load_event(k, "i")) << ";\n";
+      body_acc(o, "    ", "");
+      o << "  }\n";
+      acc_finish(o);
+      block_reduce(o);
+    };
     // ---- ragged segments: one block per segment ----
     s << "extern \"C\" __global__ void __launch_bounds__(MF_BLOCK) " << out.entry << "_segments(const " << DT
       << "* __restrict__ data, mf_u64 stride, const mf_u64* __restrict__ seg_begin,"
       << " const unsigned* __restrict__ seg_count, const mf_args* __restrict__ args,"
       << " double* __restrict__ out) {\n";
-    load_table(s);
     s << "  const unsigned seg = blockIdx.x;\n  const mf_u64 first = seg_begin[seg];\n"
-      << "  const mf_u64 cnt = seg_count[seg];\n  const mf_args& P = args[seg];\n";
-    prologue(s, "P.");
-    acc_decl(s);
-    s << "  for (mf_u64 i = threadIdx.x; i < cnt; i += MF_BLOCK) {\n";
-    for (int k : out.used_inputs)
-      s << "    const " << XT << " x" << k << " = " << input_value("__ldg(data + (mf_u64)" + std::to_string(k) +
-                                                                   " * stride + first + i)")
-        << ";\n";
-    body_acc(s, "    ", "");
-    s << "  }\n";
-    acc_finish(s);
-    block_reduce(s);
+      << "  const unsigned cnt = seg_count[seg];\n  const mf_args& P = args[seg];\n";
+    segment_work(s);
     s << R"CUDA(  for (int j = threadIdx.x; j < MF_NOUT; j += MF_BLOCK)
     out[(mf_u64)seg * MF_NOUT + j] = mf_dw_to_double(mf_dw_make(mf_blk[j].x, mf_blk[j].y));
 }
@@ -2364,22 +2388,11 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
     s << "extern \"C\" __global__ void __launch_bounds__(MF_BLOCK) " << out.entry
       << "_multi(const mf_seg* __restrict__ segs, const mf_args* __restrict__ args,"
       << " float2* __restrict__ partials) {\n";
-    load_table(s);
     s << "  const mf_seg S = segs[blockIdx.x];\n"
       << "  const " << DT << "* __restrict__ data = static_cast<const " << DT << "*>(S.data);\n"
       << "  const mf_u64 stride = S.stride, first = S.first;\n  const unsigned cnt = S.count;\n"
       << "  const mf_args& P = args[S.req];\n";
-    prologue(s, "P.");
-    acc_decl(s);
-    s << "  for (unsigned i = threadIdx.x; i < cnt; i += MF_BLOCK) {\n";
-    for (int k : out.used_inputs)
-      s << "    const " << XT << " x" << k << " = " << input_value("__ldg(data + (mf_u64)" + std::to_string(k) +
-                                                                   " * stride + first + i)")
-        << ";\n";
-    body_acc(s, "    ", "");
-    s << "  }\n";
-    acc_finish(s);
-    block_reduce(s);
+    segment_work(s);
     s << R"CUDA(  for (int j = threadIdx.x; j < MF_NOUT; j += MF_BLOCK) partials[(mf_u64)S.row * MF_NOUT + j] = mf_blk[j];
 }
 )CUDA";
