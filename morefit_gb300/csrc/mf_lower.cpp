@@ -237,12 +237,23 @@ int Parser::variable(const std::string& id) {
   fail("unknown variable '" + id + "'");
 }
 
-int Dag::intern(const Node& n) {
-  char key[160];
+// A node's fields as bytes.
+static std::string node_key(const Node& n) {
   uint64_t bits;
   std::memcpy(&bits, &n.value, sizeof bits);
-  std::snprintf(key, sizeof key, "%d|%d|%llx|%d|%d|%d|%d", int(n.op), int(n.cmp), (unsigned long long)bits, n.index,
-                n.a, n.b, n.c);
+  const uint64_t k[4] = {(uint64_t(n.op) << 8) | uint64_t(n.cmp), bits,
+                         (uint64_t(uint32_t(n.index)) << 32) | uint32_t(n.a),
+                         (uint64_t(uint32_t(n.b)) << 32) | uint32_t(n.c)};
+  return std::string(reinterpret_cast<const char*>(k), sizeof k);
+}
+
+int Dag::find(const Node& n) const {
+  auto it = table_.find(node_key(n));
+  return it != table_.end() ? it->second : -1;
+}
+
+int Dag::intern(const Node& n) {
+  const std::string key = node_key(n);
   auto it = table_.find(key);
   if (it != table_.end()) return it->second;
   nodes_.push_back(n);
@@ -312,6 +323,13 @@ int Dag::binary(Op op, int a, int b) {
   n.a = a;
   n.b = b;
   n.uniform = x.uniform && y.uniform;
+  if (op == Op::Add || op == Op::Mul) {  // the same sum or product with its operands exchanged
+    Node m = n;
+    m.a = b;
+    m.b = a;
+    const int known = find(m);
+    if (known >= 0) return known;
+  }
   return intern(n);
 }
 
@@ -850,11 +868,16 @@ __device__ __forceinline__ mf_dw mf_dw_exp(mf_dw a, const float2* __restrict__ t
 // a^b = exp(b ln|a|) in double-float. a < 0: for integer b the sign follows
 // b's parity, otherwise NaN; a = 0: 0 for b > 0, +inf for b < 0; b = 0: 1
 // (also for a NaN). Relative error ~|b ln a| 2^-46.
-__device__ __forceinline__ mf_dw mf_dw_pow(mf_dw a, mf_dw b, const float4* __restrict__ ltab,
-                                           const float2* __restrict__ etab) {
+// `la` is ln|a| (mf_dw_logabs), which the powers of one base and its logarithm share.
+__device__ __forceinline__ mf_dw mf_dw_logabs(mf_dw a, const float4* __restrict__ tab) {
+  return mf_dw_log(a.h < 0.0f ? mf_dw_neg(a) : a, tab);
+}
+__device__ __forceinline__ mf_dw mf_dw_log_of(mf_dw a, mf_dw la) {  // ln a from ln|a|
+  return a.h < 0.0f ? mf_dw_make(__uint_as_float(0x7fc00000u), 0.0f) : la;
+}
+__device__ __forceinline__ mf_dw mf_dw_pow(mf_dw a, mf_dw b, mf_dw la, const float2* __restrict__ etab) {
   const bool neg = a.h < 0.0f;
-  const mf_dw aa = neg ? mf_dw_neg(a) : a;
-  mf_dw r = mf_dw_exp(mf_dw_mul(b, mf_dw_log(aa, ltab)), etab);
+  mf_dw r = mf_dw_exp(mf_dw_mul(b, la), etab);
   // integer b and its parity from the significand bits (|v| < 2^23: v + 2^23
   // holds v's integer part in its last bits; |v| >= 2^23 is an integer)
   const float bh = fabsf(b.h), bl = fabsf(b.l);
@@ -1619,6 +1642,29 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
     }
     bool has_addu = false;
     for (int u : addu) has_addu = has_addu || u >= 0;
+    // Double-float REDUCE bodies: the powers of one per-event base, and its
+    // logarithm, share ln|base| (a third of a pow's instructions): base ->
+    // the first statement that uses it, which defines la<base>.
+    std::map<int, int> pow_base;
+    if (ar == Ar::DW && dw_exp) {
+      for (size_t i = 0; i < ns.size(); i++)
+        if (live[i] && !ns[i].uniform && ns[i].op == Op::Pow && !ns[ns[i].a].uniform) pow_base[ns[i].a] = -1;
+      for (size_t i = 0; i < ns.size(); i++)
+        if (live[i] && !ns[i].uniform && !skip[i] && (ns[i].op == Op::Pow || ns[i].op == Op::Log)) {
+          auto it = pow_base.find(ns[i].a);
+          if (it != pow_base.end() && it->second < 0) it->second = int(i);
+        }
+    }
+    auto rcp_of = [&](int a) {  // the live per-event reciprocal of node a, or -1
+      for (size_t i = 0; i < ns.size(); i++)
+        if (live[i] && !ns[i].uniform && ns[i].op == Op::Rcp && ns[i].a == a) return int(i);
+      return -1;
+    };
+    auto logabs = [&](int id) -> std::string {  // defined with its first use
+      const int b = ns[id].a;
+      if (pow_base.at(b) != id) return "";
+      return "const mf_dw la" + std::to_string(b) + " = mf_dw_logabs(" + eref(b) + ", mf_logtab); ";
+    };
     auto estmt = [&](int id) -> std::string {
       const Node& n = ns[id];
       if (ar == Ar::F32S && dnode[id])
@@ -1682,8 +1728,16 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
         case Op::Mul: return lhs + "mf_dw_mul(" + A + ", " + B + ");";
         case Op::Div: return lhs + "mf_dw_mul(" + A + ", mf_dw_rcp(" + B + "));";
         case Op::Neg: return lhs + "mf_dw_neg(" + A + ");";
-        case Op::Rcp: return lhs + "mf_dw_rcp(" + A + ");";
-        case Op::Log: return lhs + "mf_dw_log(" + A + ", mf_logtab);";
+        case Op::Rcp:
+          // 1/a^2 where 1/a is there already: its square
+          if (ns[n.a].op == Op::Mul && ns[n.a].a == ns[n.a].b) {
+            const int r = rcp_of(ns[n.a].a);
+            if (r >= 0 && r < id && !skip[r]) return lhs + "mf_dw_mul(" + eref(r) + ", " + eref(r) + ");";
+          }
+          return lhs + "mf_dw_rcp(" + A + ");";
+        case Op::Log:
+          if (pow_base.count(n.a)) return logabs(id) + lhs + "mf_dw_log_of(" + A + ", la" + std::to_string(n.a) + ");";
+          return lhs + "mf_dw_log(" + A + ", mf_logtab);";
         case Op::Sqrt: return lhs + "mf_dw_sqrt(" + A + ");";
         case Op::Sin:
         case Op::Cos: {
@@ -1696,7 +1750,10 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
           return "mf_dw " + sn + ", " + cn + "; mf_dw_sincos(" + A + ", &" + sn + ", &" + cn + ");";
         }
         case Op::Pow:
-          if (dw_exp) return lhs + "mf_dw_pow(" + A + ", " + B + ", mf_logtab, mf_exptab);";
+          if (dw_exp && pow_base.count(n.a))
+            return logabs(id) + lhs + "mf_dw_pow(" + A + ", " + B + ", la" + std::to_string(n.a) + ", mf_exptab);";
+          if (dw_exp)  // a parameter-only base
+            return lhs + "mf_dw_pow(" + A + ", " + B + ", mf_dw_logabs(" + A + ", mf_logtab), mf_exptab);";
           return lhs + "mf_dw_from_double(pow(" + D(A) + ", " + D(B) + "));";
         case Op::Exp:
           if (dw_exp) return lhs + "mf_dw_exp(" + A + ", mf_exptab);";

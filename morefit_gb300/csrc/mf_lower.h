@@ -64,6 +64,7 @@ class Dag {
   void eval_all(const double* params, size_t np, std::vector<double>& vals) const;
 
  private:
+  int find(const Node& n) const;  // an existing node like n, or -1
   int intern(const Node& n);
   std::vector<Node> nodes_;
   std::map<std::string, int> table_;

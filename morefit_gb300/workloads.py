@@ -23,6 +23,8 @@ the covariance to -2 H^-1 F H^-1 (fitter.hh:894-943). ``fisher()`` and
 """
 from __future__ import annotations
 
+import ast
+import functools
 import json
 import re
 from pathlib import Path
@@ -50,6 +52,30 @@ def weighted_covariance(hessian: np.ndarray, fisher: np.ndarray) -> np.ndarray:
     (sum w d2 log p)^-1 in the fitter's -2 ln L convention."""
     hinv = np.linalg.inv(np.asarray(hessian, dtype=np.float64))
     return -2.0 * hinv @ np.asarray(fisher, dtype=np.float64) @ hinv
+
+
+@functools.lru_cache(maxsize=1024)
+def _definition(text: str):
+    """What a parameter buffer's expression computes, as a comparable value in
+    which the operand order of a sum or product does not matter (exactly the
+    same double either way); the text itself where it holds a conditional."""
+    if "?" in text:
+        return text
+
+    def key(n):
+        if isinstance(n, ast.BinOp):
+            pair = [key(n.left), key(n.right)]
+            commutes = isinstance(n.op, (ast.Add, ast.Mult))
+            return (type(n.op).__name__, *(sorted(pair, key=repr) if commutes else pair))
+        if isinstance(n, ast.UnaryOp):
+            return (type(n.op).__name__, key(n.operand))
+        if isinstance(n, ast.Call):
+            return (n.func.id, *map(key, n.args))
+        return n.value if isinstance(n, ast.Constant) else n.id
+    try:
+        return key(ast.parse(text, mode="eval").body)
+    except (SyntaxError, AttributeError):
+        return text
 
 
 class Likelihood:
@@ -313,9 +339,16 @@ class Likelihood:
                 or list(h["params"][nth:]) != [n for n, _ in hbuf] or g["params"][:nth] != h["params"][:nth]:
             return None
 
+        # The Hessian's parameter buffers get names of their own, except those
+        # whose definition the gradient's buffers already hold: the two texts
+        # then share the subexpressions built on them (the Crystal Ball's
+        # powers and exponentials, the P-wave density's dot product).
+        known = {_definition(e): n for n, e in gbuf}
+        names = {n: known.get(_definition(e), n.replace("morefit_", "mfh_")) for n, e in hbuf}
+
         def ren(e):
-            return re.sub(r"\bmorefit_parambuffer_(\d+)\b", r"mfh_parambuffer_\1", e)
-        hb = [(ren(n), ren(e)) for n, e in hbuf]
+            return re.sub(r"\bmorefit_parambuffer_\d+\b", lambda m: names.get(m.group(0), m.group(0)), e)
+        hb = [(names[n], ren(e)) for n, e in hbuf if names[n].startswith("mfh_")]
         params = list(g["params"]) + [n for n, _ in hb]
         exprs = list(g["exprs"]) + [ren(e) for e in h["exprs"]]
         defs = dict(gbuf)
