@@ -236,6 +236,7 @@ FoldResult fold_columns(const Dag& dag, const std::vector<int>& roots, const std
   }
   // The rewritten DAG: its input indices are the prepared columns.
   auto work = std::make_unique<Dag>(dag.input_names(), dag.param_names());
+  work->share_exchanged = dag.share_exchanged;
   Dag& d2 = *work;
   std::vector<int> umemo(N, -1);
   std::vector<K> kind(N, K::Dead);

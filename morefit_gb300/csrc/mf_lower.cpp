@@ -323,7 +323,7 @@ int Dag::binary(Op op, int a, int b) {
   n.a = a;
   n.b = b;
   n.uniform = x.uniform && y.uniform;
-  if (op == Op::Add || op == Op::Mul) {  // the same sum or product with its operands exchanged
+  if (share_exchanged && (op == Op::Add || op == Op::Mul)) {  // the same sum or product with its operands exchanged
     Node m = n;
     m.a = b;
     m.b = a;
@@ -1231,6 +1231,9 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
     in_names = gen->dims;
   }
   Dag dag(in_names, params);
+  // FP32 arithmetic keeps the text's own operations: which products the
+  // compiler fuses into sums, and so the last bit, follows them
+  dag.share_exchanged = elem == Elem::F64 && !f32_arith;
   std::vector<int> roots0;
   for (auto& e : exprs) roots0.push_back(dag.parse(e));
   std::vector<int> source_inputs;
@@ -2260,15 +2263,15 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
     // evaluation: the P-wave Hessian's eight warps per SM keep 18 KB of loads
     // in flight without it, which is 2.8 TB/s) and the next events fit in
     // registers beside the accumulators at the same blocks per SM. Lone calls,
-    // 1M events (S+P FP32: 3M), without and with: P wave gradient 30.4 / 27.3
-    // us, value 26.5 / 25.9, Hessian 54.8 / 45.5, S+P gradient 52.6 / 45.6,
-    // value 33.8 / 32.4, P wave FP32 gradient 21.5 / 20.2, mass FP32 22.4 /
-    // 21.5; but P wave FP32 Hessian 30.9 / 34.2 and S+P FP32 gradient 44.4 /
-    // 50.1 (a block per SM fewer), and the S+P Hessian spills. Batched
-    // evaluations overlap their neighbours instead and keep the registers
-    // (P-wave gradient, 64 points of 100k events: 175 without, 190 with).
-    const bool lone_prefetch = !out.pipelined && NC > 0 &&
-                               (ar == Ar::DW ? M <= kAccRegMax : ar != Ar::F64 && M <= 16 && NC * V <= 40);
+    // 1M events, without and with: P wave gradient 30.4 / 27.3 us, value 26.5
+    // / 25.9, Hessian 54.8 / 45.5, S+P gradient 52.6 / 45.6, value 33.8 /
+    // 32.4; the S+P Hessian spills. FP32 kernels keep the plain loop: they are
+    // nearer the copy rate (S+P gradient, 3M: 44.4 us without, 50.1 with), and
+    // which of their products the compiler fuses into a sum, and so their last
+    // bit, follows the loop's form. Batched evaluations overlap their
+    // neighbours instead and keep the registers (P-wave gradient, 64 points of
+    // 100k events: 175 without, 190 with).
+    const bool lone_prefetch = !out.pipelined && NC > 0 && ar == Ar::DW && M <= kAccRegMax;
     std::ostringstream lone_work, part_work;
     block_work(lone_work, lone_prefetch);
     block_work(part_work, false);
@@ -2393,8 +2396,9 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
     // warps hide little latency. Toys of 2000 P-wave events, one call, plain
     // and so: value of 1 toy 52 / 37 us, of 1000 144 / 112, of 4096 388 / 315;
     // F, gradient and Hessian of 1000 toys 311 / 304. Kernels whose partials
-    // fill the registers (more than kAccRegMax outputs) keep the plain loop.
-    const bool seg_prefetch = M <= kAccRegMax;
+    // fill the registers (more than kAccRegMax outputs) and FP32 ones keep the
+    // plain loop (see lone_prefetch).
+    const bool seg_prefetch = ar == Ar::DW && M <= kAccRegMax;
     auto segment_work = [&](std::ostringstream& o) {
       auto load_event = [&](int k, const std::string& at) {
         return "__ldg(data + (mf_u64)" + std::to_string(k) + " * stride + first + " + at + ")";

@@ -51,7 +51,9 @@ class Dag {
   int input_count() const { return int(inputs_.size()); }
   const std::vector<std::string>& input_names() const { return inputs_; }
   const std::vector<std::string>& param_names() const { return params_; }
-  // Node constructors with local simplification and hash-consing.
+  // Node constructors with local simplification and hash-consing; with
+  // share_exchanged, a + b and b + a (a * b and b * a) are one node.
+  bool share_exchanged = true;
   int constant(double v);
   int unary(Op op, int a);
   int binary(Op op, int a, int b);

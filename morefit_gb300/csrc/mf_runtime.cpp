@@ -943,6 +943,15 @@ int mf_kernel_build(mf_context* c, const mf_kernel_desc* d, mf_kernel** out) {
   // evaluation with one block of 256 threads per SM against 27.2 us with two.
   if (dw && d->n_outputs > 16)
     k->blocks_per_sm = std::min(k->blocks_per_sm, std::max(1, 256 / int(k->lowered.block)));
+  // FP32 kernels of eight outputs and more: at most 16 warps per SM. Their
+  // compensated FP32 partials round with the partition, so sums of large
+  // datasets follow the grid at 1e-9, and it should not follow a register
+  // count. Two blocks of 256 against the four that fit the mass Hessian (1M
+  // events): 23.2 against 23.8 us lone, 6.9 against 7.8 batched; the Crystal
+  // Ball gradient (1M) 30.9 against 28.8 and 12.0 against 12.6.
+  const bool fp32 = d->kind == MF_KERNEL_REDUCE && (d->elem_type == MF_F32 || (d->flags & MF_FLAG_F32_ARITH));
+  if (fp32 && d->n_outputs >= 8)
+    k->blocks_per_sm = std::min(k->blocks_per_sm, std::max(1, 512 / int(k->lowered.block)));
   if (dw) k->desc = std::make_unique<DescCopy>(d);
   c->refs++;
   k->holds_ref = true;

@@ -342,8 +342,9 @@ class Likelihood:
         # The Hessian's parameter buffers get names of their own, except those
         # whose definition the gradient's buffers already hold: the two texts
         # then share the subexpressions built on them (the Crystal Ball's
-        # powers and exponentials, the P-wave density's dot product).
-        known = {_definition(e): n for n, e in gbuf}
+        # powers and exponentials, the P-wave density's dot product). Not in
+        # FP32 arithmetic, whose last bit follows the text's own operations.
+        known = {_definition(e): n for n, e in gbuf} if self.kernelT == np.float64 else {}
         names = {n: known.get(_definition(e), n.replace("morefit_", "mfh_")) for n, e in hbuf}
 
         def ren(e):
