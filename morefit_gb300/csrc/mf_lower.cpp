@@ -689,65 +689,76 @@ __device__ __forceinline__ mf_dw mf_dw_split_rn(double x) {
                              low ? 0x1p-64f : 1.0f);
   return mf_dw_make(h, __uint_as_float(__float_as_uint(lm) | (sign ^ (L < 0 ? 0x80000000u : 0u))));
 }
-// h + l as an FP64 value with integer operations only: h's significand
-// extended by l's bits down to the double's last place (l's bits below it
-// are dropped, an error below one unit in the last place). The pair is
-// renormalized first; zero or subnormal h gives a signed zero (an absolute
-// error below 2^-125), inf and NaN carry over.
+// A normalized pair (|l| <= ulp(h)/2, as every operation here returns) as an
+// FP64 value without the FP64 pipe: the double of h from its bits, moved by l
+// in units of the double's last place (one exact scaling and one conversion to
+// an integer, |l| <= 2^28 units, rounded to nearest) as an integer step of the
+// bit pattern, which cannot leave h's binade upwards. Powers of two, whose
+// lower neighbours are half as far apart, magnitudes below 2^-75, zero, inf
+// and NaN take the general form, out of line: zero or subnormal h gives a
+// signed zero (an absolute error below 2^-125), inf and NaN carry over.
+__device__ __noinline__ double mf_dw_to_double_rare(float h, float l) {
+  const unsigned hb = __float_as_uint(h), sign = hb & 0x80000000u;
+  const int eh = (int)((hb >> 23) & 0xffu);
+  const float up = sign ? -l : l;  // away from zero
+  // times 2^(179 - eh), twice that below a power of two, in two exact steps
+  const int sh = 179 - eh + ((hb & 0x7fffffu) == 0u && up < 0.0f ? 1 : 0), s1 = sh / 2;
+  const float units = __fmul_rn(__fmul_rn(up, __uint_as_float((unsigned)(127 + s1) << 23)),
+                                __uint_as_float((unsigned)(127 + sh - s1) << 23));
+  const int li = eh != 0 && eh != 255 ? __float2int_rn(units) : 0;
+  long long bits = ((long long)(hb & 0x7fffffffu) << 29) + (896ll << 52) + (long long)li;
+  if (eh == 0) bits = 0;
+  if (eh == 255) bits = (0x7ffll << 52) | ((hb & 0x7fffffu) ? (1ll << 51) : 0ll);
+  return __longlong_as_double(bits | ((long long)sign << 32));
+}
 __device__ __forceinline__ double mf_dw_to_double_bits(mf_dw a) {
-  a = mf_fast_two_sum(a.h, a.l);
-  const unsigned hb = __float_as_uint(a.h), lb = __float_as_uint(a.l);
-  const int eh = (int)((hb >> 23) & 0xffu), el = (int)((lb >> 23) & 0xffu);
-  const int k = 29 + el - eh;  // scale of l's significand in units of the double's last place (<= 5)
-  if (eh == 0 || eh == 255)
-    return __longlong_as_double((long long)(((unsigned long long)(hb >> 31) << 63) |
-                                            (eh ? (0x7ffull << 52) | ((hb & 0x7fffffu) ? (1ull << 51) : 0ull) : 0ull)));
-  unsigned long long M = (unsigned long long)((hb & 0x7fffffu) | 0x800000u) << 29;
-  int E = eh;
-  if (el != 0) {
-    const unsigned long long ml = (lb & 0x7fffffu) | 0x800000u;
-    const unsigned long long v = k >= 0 ? (ml << k) : (k > -40 ? (ml >> -k) : 0ull);
-    if ((hb ^ lb) >> 31) {
-      M -= v;
-      if (M < (1ull << 52)) { M <<= 1; E -= 1; }
-    } else {
-      M += v;
-      if (M >= (1ull << 53)) { M >>= 1; E += 1; }
-    }
-  }
-  return __longlong_as_double((long long)(((unsigned long long)(hb >> 31) << 63) |
-                                          ((unsigned long long)(E + 896) << 52) | (M & 0xfffffffffffffull)));
+  const unsigned hb = __float_as_uint(a.h), e = hb & 0x7f800000u, sign = hb & 0x80000000u;
+  if ((hb & 0x7fffffu) == 0u || e - (52u << 23) >= (203u << 23)) return mf_dw_to_double_rare(a.h, a.l);
+  // l * 2^(179 - eh), negated where h is negative
+  const int li = __float2int_rn(__fmul_rn(a.l, __uint_as_float(((306u << 23) - e) ^ sign)));
+  const unsigned long long h = ((unsigned long long)((((hb & 0x7fffffffu) >> 3) + 0x38000000u) | sign) << 32) | (hb << 29);
+  return __longlong_as_double((long long)h + (long long)li);
 }
-__device__ __forceinline__ mf_dw mf_dw_mulf(mf_dw a, float b) {
-  const float p = __fmul_rn(a.h, b);
-  return mf_fast_two_sum(p, __fmaf_rn(a.l, b, __fmaf_rn(a.h, b, -p)));
-}
-// Square root: the correctly rounded FP32 root s of a.h, corrected by the
-// series sqrt(s^2 + r) = s + d - d^2/(2s) + ..., d = r/(2s). d reaches
-// 2^-23 s, so the residual r = a - s^2 (s^2 exact by FMA) and d are kept as
-// double-float values; the next term, d^3/(2s^2), is below 2^-70 s.
-// sqrt(0) = 0, negative or NaN -> NaN, +inf -> +inf.
+// Square root: s = a.h / sqrt(a.h) and h = 1 / (2 sqrt(a.h)) in FP32, each
+// corrected once (Goldschmidt's iteration), then the series sqrt(s^2 + r) =
+// s + d - d^2/(2s) + ..., d = r/(2s). d reaches 2^-23 s, so the residual
+// r = a - s^2 (s^2 exact by FMA) and d are kept as double-float values, d by
+// the reciprocal h and one correction; the next term, d^3/(2s^2), is below
+// 2^-70 s. sqrt(0) = 0, negative or NaN -> NaN, +inf -> +inf.
 __device__ __forceinline__ mf_dw mf_dw_sqrt(mf_dw a) {
   if (!(a.h > 0.0f) || a.h == __int_as_float(0x7f800000))
     return mf_dw_make(a.h == 0.0f ? 0.0f : (a.h > 0.0f ? a.h : __int_as_float(0x7fc00000)), 0.0f);
-  const float s = __fsqrt_rn(a.h);
+  const float y = rsqrtf(a.h);
+  const float s0 = __fmul_rn(a.h, y), h0 = __fmul_rn(0.5f, y);
+  const float c = __fmaf_rn(-s0, h0, 0.5f);
+  const float s = __fmaf_rn(s0, c, s0), h = __fmaf_rn(h0, c, h0);
   const float p = __fmul_rn(s, s);
   const float pe = __fmaf_rn(s, s, -p);
   // a.h - p is exact (Sterbenz); the rest of the residual in double-float
-  const mf_dw r = mf_dw_add(mf_two_sum(__fsub_rn(a.h, p), -pe), mf_dw_make(a.l, 0.0f));
-  const float s2 = __fadd_rn(s, s);
-  const float dh = __fdiv_rn(r.h, s2);
-  const float dl = __fdiv_rn(__fadd_rn(__fmaf_rn(-dh, s2, r.h), r.l), s2);
-  const float q = __fdiv_rn(__fmul_rn(dh, dh), s2);
+  const mf_dw r0 = mf_two_sum(__fsub_rn(a.h, p), -pe), r = mf_two_sum(r0.h, a.l);
+  const float rl = __fadd_rn(r0.l, r.l);
+  const float dh = __fmul_rn(__fadd_rn(r.h, rl), h);
+  const float dl = __fmul_rn(__fadd_rn(__fmaf_rn(-dh, __fadd_rn(s, s), r.h), rl), h);
+  const float q = __fmul_rn(__fmul_rn(dh, dh), h);
   const mf_dw t = mf_fast_two_sum(s, dh);
   return mf_fast_two_sum(t.h, __fadd_rn(t.l, __fsub_rn(dl, q)));
+}
+// c + x * q for |x q| < |c|, not renormalized
+__device__ __forceinline__ mf_dw mf_dw_horner(mf_dw c, mf_dw x, mf_dw q) {
+  const float p = __fmul_rn(x.h, q.h);
+  const float e = __fmaf_rn(x.h, q.l, __fmaf_rn(x.l, q.h, __fmaf_rn(x.h, q.h, -p)));
+  const float s = __fadd_rn(c.h, p);
+  return mf_dw_make(s, __fadd_rn(__fsub_rn(p, __fsub_rn(s, c.h)), __fadd_rn(c.l, e)));
 }
 // sin and cos of a double-float. a = k*(pi/2) + r, |r| <~ pi/4, by a
 // four-part Cody-Waite reduction: pi/2 = C1 + C2 + C3 + C4 with C1 and C2 of
 // 12 significant bits (k*C1, k*C2 exact for |k| < 2^12) and a remainder below
 // 4e-22. sin r and cos r are their Taylor series, the terms above 2^-26 in
 // double-float (Horner), the rest in FP32; the first omitted term is below
-// 2e-16 relative. Arguments beyond |a| = 6000 (and inf/NaN) use FP64.
+// 2e-16 relative. A Horner step adds a product to a coefficient at least 16
+// times as large, so it needs neither an ordered sum nor a renormalized
+// result: nine operations (mf_dw_horner). Arguments beyond |a| = 6000 (and
+// inf/NaN) use FP64.
 __device__ __forceinline__ void mf_dw_sincos(mf_dw a, mf_dw* sn, mf_dw* cs) {
   if (!(fabsf(a.h) <= 6000.0f)) {
     const double x = mf_dw_to_double(a);
@@ -765,19 +776,21 @@ __device__ __forceinline__ void mf_dw_sincos(mf_dw a, mf_dw* sn, mf_dw* cs) {
   const float z = r2.h;
   // sin r = r + r^3 (c3 + r^2 (c5 + r^2 (c7 + r^2 (c9 + r^2 T)))), c_n = (-1)^((n-1)/2) / n!
   const float T = __fmaf_rn(z, __fmaf_rn(z, -0x1.ae7f3ep-41f, 0x1.612462p-33f), -0x1.ae6456p-26f);
-  mf_dw q = mf_dw_add(mf_dw_make(0x1.71de3ap-19f, 0x1.55b1ccp-45f), mf_dw_mulf(r2, T));
-  q = mf_dw_add(mf_dw_make(-0x1.a01a02p-13f, 0x1.7f97fap-39f), mf_dw_mul(r2, q));
-  q = mf_dw_add(mf_dw_make(0x1.111112p-7f, -0x1.dddddep-32f), mf_dw_mul(r2, q));
-  q = mf_dw_add(mf_dw_make(-0x1.555556p-3f, 0x1.555556p-28f), mf_dw_mul(r2, q));
-  const mf_dw sr = mf_dw_add(r, mf_dw_mul(mf_dw_mul(r, r2), q));
+  mf_dw q = mf_dw_horner(mf_dw_make(0x1.71de3ap-19f, 0x1.55b1ccp-45f), r2, mf_dw_make(T, 0.0f));
+  q = mf_dw_horner(mf_dw_make(-0x1.a01a02p-13f, 0x1.7f97fap-39f), r2, q);
+  q = mf_dw_horner(mf_dw_make(0x1.111112p-7f, -0x1.dddddep-32f), r2, q);
+  q = mf_dw_horner(mf_dw_make(-0x1.555556p-3f, 0x1.555556p-28f), r2, q);
+  mf_dw sr = mf_dw_horner(r, mf_dw_mul(r, r2), q);
+  sr = mf_fast_two_sum(sr.h, sr.l);
   // cos r = 1 + r^2 (c2 + r^2 (c4 + r^2 (c6 + r^2 (c8 + r^2 (c10 + r^2 T2))))), c_n = (-1)^(n/2) / n!
   const float T2 = __fmaf_rn(z, __fmaf_rn(z, 0x1.ae7f3ep-45f, -0x1.93974ap-37f), 0x1.1eed8ep-29f);
-  mf_dw u = mf_dw_add(mf_dw_make(-0x1.27e4fcp-22f, 0x1.10ec14p-47f), mf_dw_mulf(r2, T2));
-  u = mf_dw_add(mf_dw_make(0x1.a01a02p-16f, -0x1.7f97fap-42f), mf_dw_mul(r2, u));
-  u = mf_dw_add(mf_dw_make(-0x1.6c16c2p-10f, 0x1.27d27ep-35f), mf_dw_mul(r2, u));
-  u = mf_dw_add(mf_dw_make(0x1.555556p-5f, -0x1.555556p-30f), mf_dw_mul(r2, u));
-  u = mf_dw_add(mf_dw_make(-0.5f, 0.0f), mf_dw_mul(r2, u));
-  const mf_dw cr = mf_dw_add(mf_dw_make(1.0f, 0.0f), mf_dw_mul(r2, u));
+  mf_dw u = mf_dw_horner(mf_dw_make(-0x1.27e4fcp-22f, 0x1.10ec14p-47f), r2, mf_dw_make(T2, 0.0f));
+  u = mf_dw_horner(mf_dw_make(0x1.a01a02p-16f, -0x1.7f97fap-42f), r2, u);
+  u = mf_dw_horner(mf_dw_make(-0x1.6c16c2p-10f, 0x1.27d27ep-35f), r2, u);
+  u = mf_dw_horner(mf_dw_make(0x1.555556p-5f, -0x1.555556p-30f), r2, u);
+  u = mf_dw_horner(mf_dw_make(-0.5f, 0.0f), r2, u);
+  u = mf_dw_horner(mf_dw_make(1.0f, 0.0f), r2, u);
+  const mf_dw cr = mf_fast_two_sum(u.h, u.l);
   const int quad = ((int)k) & 3;
   const mf_dw s0 = (quad & 1) ? cr : sr, c0 = (quad & 1) ? sr : cr;
   *sn = (quad & 2) ? mf_dw_neg(s0) : s0;
@@ -1274,7 +1287,9 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
 
   LoweredKernel out;
   out.entry = "mf_" + std::string(kind == Kind::Reduce ? "reduce" : kind == Kind::Store ? "store" : "generate");
-  out.block = kind == Kind::Generate ? 128 : 256;
+  // GENERATE and STORE: small blocks, whose ends leave less of an SM idle
+  // (S+P-wave precompute, 1M events: 71.8 us in blocks of 256, 68.9 of 128)
+  out.block = kind == Kind::Reduce ? 256 : 128;
   out.vec = (kind == Kind::Generate) ? 1 : (st32 ? 4 : 2);
   if (kind == Kind::Reduce) {
     out.pipelined = !direct_loads;
@@ -1781,7 +1796,13 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
       // Event-only precompute in double-float: inputs split with rounding
       // and outputs joined by integer operations (the FP64 pipe, 1/64 of the
       // FP32 rate on GB300, is not used per event), parameter-only values
-      // evaluated in FP64 once per thread.
+      // evaluated in FP64 once per thread. Bound by instruction issue, most
+      // of it on the half-rate integer pipe: the P wave's 1M events took 67.6
+      // us at about 1900 instructions per event and take 43.3 at about 1200
+      // (136 MB are 20 us at the copy rate); the S+P wave 99.2 and 68.9. What
+      // went: the divisions of the square root, the ordered and renormalized
+      // sums of the sine's and cosine's Horner steps, and the shifts and
+      // special cases of joining a pair.
       std::set<int> uni;
       for (size_t i = 0; i < ns.size(); i++) {
         if (!live[i] || ns[i].uniform || ns[i].op == Op::Input) continue;
