@@ -635,6 +635,11 @@ __device__ __forceinline__ void mf_dw_acc_mul(mf_dw& a, mf_dw x, mf_dw y) {
   a.h = s.h;
   a.l = __fadd_rn(a.l, __fadd_rn(s.l, e));
 }
+// x * y as such a sum begins: acc_mul onto zero
+__device__ __forceinline__ mf_dw mf_dw_prod(mf_dw x, mf_dw y) {
+  const float p = __fmul_rn(x.h, y.h);
+  return mf_dw_make(p, __fmaf_rn(x.h, y.l, __fmaf_rn(x.l, y.h, __fmaf_rn(x.h, y.h, -p))));
+}
 // a += x * y for FP32 operands: the product is exact as p + e (FMA), so a
 // dot product of FP32 values accumulated this way is as accurate as one
 // computed in double-float (the compensated dot product of Ogita, Rump and
@@ -1736,8 +1741,10 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
       if (skip[id]) return "";
       auto ch = chains.find(id);
       if (ch != chains.end()) {
-        std::string c = "mf_dw e" + std::to_string(id) + "; { mf_dw t_ = mf_dw_make(0.0f, 0.0f);";
-        for (auto& [ta, tb] : ch->second) c += " mf_dw_acc_mul(t_, " + eref(ta) + ", " + eref(tb) + ");";
+        std::string c = "mf_dw e" + std::to_string(id) + "; {";
+        for (auto& [ta, tb] : ch->second)
+          c += (&ta == &ch->second.front().first ? " mf_dw t_ = mf_dw_prod(" : " mf_dw_acc_mul(t_, ") + eref(ta) + ", " +
+               eref(tb) + ");";
         return c + " e" + std::to_string(id) + " = mf_dw_renorm(t_); }";
       }
       switch (n.op) {
@@ -2011,7 +2018,8 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
           o << "    " << accref(j) << " = q_; }\n";
       }
     };
-    auto acc_one = [&](std::ostringstream& o, const std::string& ind, int j) {
+    // `fresh` (double-float): the thread's first event, whose value is the partial
+    auto acc_one = [&](std::ostringstream& o, const std::string& ind, int j, bool fresh = false) {
       {
         if (logadd[j] >= 0) o << ind << "lpc" << j << "++;\n";
         if (ar == Ar::F32 && logprod[j] >= 0) {
@@ -2025,6 +2033,10 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
           o << ind << accref(j) << " += " << r << ";\n";
         else if (logprod[j] >= 0)
           o << ind << "mf_dw_logprod(lpm" << j << ", lpe" << j << ", " << eref(logprod[j]) << ");\n";
+        else if (fresh)
+          o << ind << accref(j) << " = "
+            << (fused[j].first >= 0 ? "mf_dw_prod(" + eref(fused[j].first) + ", " + eref(fused[j].second) + ")" : r)
+            << ";\n";
         else if (fused[j].first >= 0)
           o << ind << "mf_dw_acc_mul(" << accref(j) << ", " << eref(fused[j].first) << ", "
             << eref(fused[j].second) << ");\n";
@@ -2060,12 +2072,12 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
     }
     // The body and the accumulation of every output; `guard` (a condition, or
     // empty) decides whether this event counts.
-    auto body_acc = [&](std::ostringstream& o, const std::string& ind, const std::string& guard) {
+    auto body_acc = [&](std::ostringstream& o, const std::string& ind, const std::string& guard, bool fresh = false) {
       if (has_addu) o << ind << (guard.empty() ? "" : "if (" + guard + ") ") << "mf_cnt++;\n";
       auto accs = [&](const std::vector<int>& js) {
         if (js.empty()) return;
         if (!guard.empty()) o << ind << "if (" << guard << ") {\n";
-        for (int j : js) acc_one(o, guard.empty() ? ind : ind + "  ", j);
+        for (int j : js) acc_one(o, guard.empty() ? ind : ind + "  ", j, fresh);
         if (!guard.empty()) o << ind << "}\n";
       };
       if (!interleave) {
@@ -2117,9 +2129,7 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
       for (int r = M; r > 0; r -= pick[r]) v.push_back(pick[r]);
       return v;
     }();
-    auto block_reduce = [&](std::ostringstream& o) {
-      o << "  __shared__ float2 mf_part[MF_PART];\n  __shared__ float2 mf_blk[MF_NOUT];\n"
-        << "  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;\n";
+    auto warp_reduce = [&](std::ostringstream& o) {  // into row `warp` of part[]
       int j0 = 0;
       for (int n : chunks) {
         o << "  {\n    mf_dw v[" << n << "];\n";
@@ -2127,10 +2137,15 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
           o << "    v[" << c << "] = " << (j0 + c < M ? thread_dw(j0 + c) : "mf_dw_make(0.0f, 0.0f)") << ";\n";
         o << "    mf_warp_sums<" << n << ">(v, lane);\n"
           << "    const int j = " << j0 << " + lane / " << 32 / n << ";\n"
-          << "    if (lane % " << 32 / n << " == 0 && j < MF_NOUT) mf_part[warp * MF_NOUT + j] = make_float2(v[0].h, v[0].l);\n"
+          << "    if (lane % " << 32 / n << " == 0 && j < MF_NOUT) part[warp * MF_NOUT + j] = make_float2(v[0].h, v[0].l);\n"
           << "  }\n";
         j0 += n;
       }
+    };
+    auto block_reduce = [&](std::ostringstream& o) {
+      o << "  __shared__ float2 mf_part[MF_PART];\n  __shared__ float2 mf_blk[MF_NOUT];\n"
+        << "  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;\n  float2* const part = mf_part;\n";
+      warp_reduce(o);
       o << "  __syncthreads();\n"
         << "  for (int j = threadIdx.x; j < MF_NOUT; j += MF_BLOCK) {\n"
         << "    mf_dw a = mf_dw_pair(mf_part[j]);\n"
@@ -2166,15 +2181,35 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
     s << kCombine;
     const int NC = int(out.used_inputs.size());
     const std::string VT = V == 1 ? DT : pair ? "float4" : st32 ? (V == 4 ? "float4" : "float2") : "double2";
+    auto load_at = [&](int k, const std::string& at) {
+      return "__ldg(reinterpret_cast<const " + VT + "*>(data + (mf_u64)" + std::to_string(k) + " * stride + " + at + "))";
+    };
+    const char* comp[4] = {"x", "y", "z", "w"};
+    // event v of the vector loaded into l<k>
+    auto lane_of = [&](int k, int v) -> std::string {
+      const std::string l = "l" + std::to_string(k);
+      if (pair) return V == 1 ? l : "make_float2(" + l + "." + comp[2 * v] + ", " + l + "." + comp[2 * v + 1] + ")";
+      return V == 1 ? l : l + "." + comp[v];
+    };
+    // the vector's events (loaded here from src(k), or l<k> defined already)
+    auto emit_events = [&](std::ostringstream& s, const std::string& ind, const std::string& valid_base,
+                           const std::function<std::string(int)>& src, bool fresh = false) {
+      for (int k : out.used_inputs)
+        if (src) s << ind << "const " << VT << " l" << k << " = " << src(k) << ";\n";
+      for (int v = 0; v < V; v++) {
+        s << ind << "{\n";
+        for (int k : out.used_inputs)
+          s << ind << "  const " << XT << " x" << k << " = " << input_value(lane_of(k, v)) << ";\n";
+        body_acc(s, ind + "  ", valid_base + " + " + std::to_string(v) + " < n", fresh && v == 0);
+        s << ind << "}\n";
+      }
+    };
     // The per-block work of the single-evaluation and the batched entry: the
     // event loop and the block reduction. `prefetch`: a thread's next events
     // are loaded while it computes its present ones, the first before the
     // tables (the same events in the same order, so the same sums).
     auto block_work = [&](std::ostringstream& s, const bool prefetch) {
       s << "  mf_launch_dependents();  // the next evaluation may start its event loop on SMs this grid frees\n";
-      auto load_at = [&](int k, const std::string& at) {
-        return "__ldg(reinterpret_cast<const " + VT + "*>(data + (mf_u64)" + std::to_string(k) + " * stride + " + at + "))";
-      };
       if (prefetch) {
         s << "  const mf_u64 step = (mf_u64)gridDim.x * MF_BLOCK * " << V << ";\n"
           << "  mf_u64 base = ((mf_u64)blockIdx.x * MF_BLOCK + threadIdx.x) * " << V << ";\n";
@@ -2184,26 +2219,6 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
       load_table(s);
       prologue(s, "P.");
       acc_decl(s);
-      const char* comp[4] = {"x", "y", "z", "w"};
-      // event v of the vector loaded into l<k>
-      auto lane_of = [&](int k, int v) -> std::string {
-        const std::string l = "l" + std::to_string(k);
-        if (pair) return V == 1 ? l : "make_float2(" + l + "." + comp[2 * v] + ", " + l + "." + comp[2 * v + 1] + ")";
-        return V == 1 ? l : l + "." + comp[v];
-      };
-      auto emit_events = [&](const std::string& ind, const std::string& idx0, const std::string& valid_base,
-                             const std::function<std::string(int)>& src) {
-        for (int k : out.used_inputs)
-          if (src) s << ind << "const " << VT << " l" << k << " = " << src(k) << ";\n";
-        for (int v = 0; v < V; v++) {
-          s << ind << "{\n";
-          for (int k : out.used_inputs)
-            s << ind << "  const " << XT << " x" << k << " = " << input_value(lane_of(k, v)) << ";\n";
-          body_acc(s, ind + "  ", valid_base + " + " + std::to_string(v) + " < n");
-          s << ind << "}\n";
-        }
-        (void)idx0;
-      };
       if (out.pipelined && NC > 0) {
         // Persistent blocks; tile t (events [t*MF_TILE, (t+1)*MF_TILE) of every
         // column read by the body) goes to block t % gridDim.x. Thread 0 keeps
@@ -2251,7 +2266,7 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
         s << "    {\n      const int e0 = threadIdx.x * " << V << ";\n";
         std::map<int, int> colpos;
         for (int ci = 0; ci < NC; ci++) colpos[out.used_inputs[ci]] = ci;
-        emit_events("      ", "e0", "tbase + e0", [&](int k) {
+        emit_events(s, "      ", "tbase + e0", [&](int k) {
           return "*reinterpret_cast<const " + VT + "*>(sb + " + std::to_string(colpos[k]) + " * MF_TILE + e0)";
         });
         s << "    }\n    __syncthreads();\n  }\n";
@@ -2265,7 +2280,7 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
         for (int k : out.used_inputs) s << "    const " << VT << " l" << k << " = c" << k << ";\n";
         for (int k : out.used_inputs)
           s << "    c" << k << " = ahead < n ? " << load_at(k, "ahead") << " : " << VT << "();\n";
-        emit_events("    ", "base", "base", nullptr);
+        emit_events(s, "    ", "base", nullptr);
         s << "  }\n";
       } else {
         s << "  const mf_u64 step = (mf_u64)gridDim.x * MF_BLOCK * " << V << ";\n";
@@ -2273,7 +2288,7 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
         if (out.stages > 1) s << "#pragma unroll " << out.stages << "\n";
         s << "  for (mf_u64 base = ((mf_u64)blockIdx.x * MF_BLOCK + threadIdx.x) * " << V
           << "; base < n; base += step) {\n";
-        emit_events("    ", "base", "base", [&](int k) { return load_at(k, "base"); });
+        emit_events(s, "    ", "base", [&](int k) { return load_at(k, "base"); });
         s << "  }\n";
       }
       s << "  __shared__ bool am_last;\n";
@@ -2293,6 +2308,9 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
     // neighbours instead and keep the registers (P-wave gradient, 64 points of
     // 100k events: 175 without, 190 with).
     const bool lone_prefetch = !out.pipelined && NC > 0 && ar == Ar::DW && M <= kAccRegMax;
+    auto replace_all = [](std::string& t, const std::string& from, const std::string& to) {
+      for (size_t p = t.find(from); p != std::string::npos; p = t.find(from, p + to.size())) t.replace(p, from.size(), to);
+    };
     std::ostringstream lone_work, part_work;
     block_work(lone_work, lone_prefetch);
     block_work(part_work, false);
@@ -2347,9 +2365,6 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
     if (!out.pipelined) {
       const std::string tail = s.str().substr(size_t(body_mark) + lone_work.str().size());
       auto resident = [&](std::string work) {
-        auto replace_all = [](std::string& t, const std::string& from, const std::string& to) {
-          for (size_t p = t.find(from); p != std::string::npos; p = t.find(from, p + to.size())) t.replace(p, from.size(), to);
-        };
         replace_all(work, "blockIdx.x", "mf_vb");
         replace_all(work, "gridDim.x", "mf_grid");
         return "__device__ __forceinline__ void mf_rbody(const " + DT +
@@ -2380,6 +2395,61 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
       << "  // stream order, so the combine launch after the last evaluation sees every partial\n"
       << "  mf_grid_dependency_wait();\n"
       << "}\n";
+    // ---- many small evaluations in one launch ----
+    // For evaluations of less than one grid of the device, where a thread has
+    // one vector of events at most and a launch each costs the host more than
+    // the device: block (vb, q) does block vb of evaluations [q * group, ...)
+    // of the launch, one after the other, its events kept in registers while
+    // they stay the same (a scan of one dataset), one table load and one
+    // barrier for all. Each row of partials is the _part entry's, and
+    // <entry>_combine follows the same way. The evaluations' columns, sizes
+    // and parameters are the launch's own argument (constant memory).
+    // Double-float kernels only: their operations are fixed one by one, an
+    // FP32 body's last bit follows the form of the loop around it.
+    if (!out.pipelined && NC > 0 && ar == Ar::DW && M <= 16) {
+      out.batch_max = int(std::min<size_t>(64, 24576 / (32 + out.args_bytes())));
+      s << "#define MF_GROUP " << kBatchGroup << "\n"
+        << "struct mf_job { const " << DT << "* data; mf_u64 stride, n, grid; mf_args P; };\n"
+        << "struct mf_batch { mf_job job[" << out.batch_max << "]; };\n"
+        << "extern \"C\" __global__ void MF_BOUNDS " << out.entry
+        << "_batch(const __grid_constant__ mf_batch B, float2* __restrict__ partials_all, mf_u64 pstride,"
+        << " unsigned count, unsigned group) {\n"
+        << "  __shared__ float2 mf_warps[MF_GROUP][MF_BLOCK / 32 * MF_NOUT];\n"
+        << "  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;\n"
+        << "  const unsigned first = blockIdx.y * group, last = first + group < count ? first + group : count;\n"
+        << "  const mf_u64 base = ((mf_u64)blockIdx.x * MF_BLOCK + threadIdx.x) * " << V << ";\n"
+        << "  const " << DT << "* __restrict__ data = B.job[first].data;\n"
+        << "  mf_u64 stride = B.job[first].stride, n = B.job[first].n;\n";
+      for (int k : out.used_inputs)
+        s << "  " << VT << " l" << k << " = base < n ? " << load_at(k, "base") << " : " << VT << "();\n";
+      load_table(s);
+      s << "  for (unsigned e = first; e < last; e++) {\n    const mf_job& J = B.job[e];\n"
+        << "    if (blockIdx.x >= J.grid) continue;\n    const mf_args& P = J.P;\n"
+        << "    if (J.data != data || J.stride != stride || J.n != n) {  // another dataset\n"
+        << "      data = J.data; stride = J.stride; n = J.n;\n";
+      for (int k : out.used_inputs)
+        s << "      l" << k << " = base < n ? " << load_at(k, "base") << " : " << VT << "();\n";
+      s << "    }\n    float2* const part = mf_warps[e - first];\n";
+      prologue(s, "P.");
+      acc_decl(s);
+      s << "    if (base < n) {\n";
+      emit_events(s, "      ", "base", nullptr, true);
+      s << "    }\n";
+      acc_finish(s);
+      warp_reduce(s);
+      s << R"CUDA(  }
+  __syncthreads();
+  for (unsigned q = threadIdx.x; q < (last - first) * MF_NOUT; q += MF_BLOCK) {
+    const unsigned e = q / MF_NOUT, j = q - e * MF_NOUT;
+    if (blockIdx.x >= B.job[first + e].grid) continue;
+    mf_dw a = mf_dw_pair(mf_warps[e][j]);
+#pragma unroll
+    for (int w = 1; w < MF_BLOCK / 32; w++) a = mf_dw_add(a, mf_dw_pair(mf_warps[e][w * MF_NOUT + j]));
+    partials_all[(first + e) * pstride + (mf_u64)blockIdx.x * MF_NOUT + j] = make_float2(a.h, a.l);
+  }
+}
+)CUDA";
+    }
     s << "extern \"C\" __global__ void __launch_bounds__(MF_BLOCK) " << out.entry
       << "_combine(float2* __restrict__ partials_all, mf_u64 pstride, const unsigned* __restrict__ grids,"
       << " double* __restrict__ out_all, unsigned count, unsigned grid_all) {\n"

@@ -26,6 +26,8 @@ namespace mf {
 // Blocks whose partial rows a REDUCE kernel of many outputs combines first
 // (one completion counter each, behind the grid's own).
 constexpr int kCombineRows = 16;
+// Evaluations a block of the _batch entry does at most, one after the other.
+constexpr int kBatchGroup = 8;
 
 enum class Op : uint8_t {
   Const, Input, Param, Add, Sub, Mul, Neg, Rcp, Div, Exp, Log, Sqrt, Sin, Cos, Tan, Asin, Acos, Atan, Erf,
@@ -108,6 +110,7 @@ struct LoweredKernel {
   // resident_plain is the same without prefetching, in fewer registers.
   std::string resident_prefix, resident_body, resident_plain;
   std::string resident_data_type;  // element type mf_rbody reads ("float2", "double", "float")
+  int batch_max = 0;      // evaluations the _batch entry takes in one launch (0: no such entry)
   size_t smem_bytes = 0;  // dynamic shared memory of the main entry
   // REDUCE kernels: host-evaluated argument struct
   // Prepared input (REDUCE): the kernel reads `prep_cols.size()` columns that

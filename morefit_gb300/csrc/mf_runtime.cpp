@@ -295,6 +295,7 @@ struct mf_kernel {
   cudaKernel_t fn_prep = nullptr;  // REDUCE kernels reading prepared columns
   cudaKernel_t fn_part = nullptr;     // REDUCE: per-block partials only (batched evaluations)
   cudaKernel_t fn_combine = nullptr;  // REDUCE: one block per batched evaluation
+  cudaKernel_t fn_batch = nullptr;    // REDUCE: many small evaluations in one launch
   cudaKernel_t fn_multi = nullptr;    // REDUCE: segments of many datasets in one launch
   uint64_t prep_key = 0;
   int blocks_per_sm = 1;
@@ -914,6 +915,8 @@ int mf_kernel_build(mf_context* c, const mf_kernel_desc* d, mf_kernel** out) {
     MF_CUDA_TRY(cudaLibraryGetKernel(&k->fn_seg, k->lib, (k->lowered.entry + "_segments").c_str()));
   if (d->kind == MF_KERNEL_REDUCE) {
     MF_CUDA_TRY(cudaLibraryGetKernel(&k->fn_part, k->lib, (k->lowered.entry + "_part").c_str()));
+    if (k->lowered.batch_max)
+      MF_CUDA_TRY(cudaLibraryGetKernel(&k->fn_batch, k->lib, (k->lowered.entry + "_batch").c_str()));
     MF_CUDA_TRY(cudaLibraryGetKernel(&k->fn_combine, k->lib, (k->lowered.entry + "_combine").c_str()));
     MF_CUDA_TRY(cudaLibraryGetKernel(&k->fn_multi, k->lib, (k->lowered.entry + "_multi").c_str()));
   }
@@ -1433,6 +1436,24 @@ int launch_reduce(mf_kernel* k, const void* data, uint64_t stride, uint64_t n, c
   return MF_OK;
 }
 
+// The head of the generated mf_job; the argument struct follows.
+struct BatchJob {
+  const void* data;
+  uint64_t stride, n, grid;
+};
+
+// Whether evaluations of up to `maxgrid` blocks go through the _batch entry:
+// each thread then has one vector of events at most (the grid is not capped).
+// Above, the launches' own cost is hidden and their parameters, constants of
+// the launch, cost no registers. 64 points of one dataset, one call through
+// Python, a launch each against the _batch entry (us): P-wave gradient 1k
+// events 149 / 51, 20k 148 / 76, 50k 152 / 100, 100k 166 / 149, 150k 212 /
+// 188; its value 100k 147 / 100; mass gradient 1k 178 / 70, 50k 172 / 132,
+// 150k 260 / 265; S+P gradient 20k 180 / 133, 50k 191 / 193.
+bool batch_fits(const mf_kernel* k, int maxgrid) {
+  return k->fn_batch && maxgrid < k->ctx->num_sms * k->blocks_per_sm;
+}
+
 // Batched evaluations in chunks of up to kChunk: evaluation e of a chunk
 // writes its per-block partials to slot e of the context's partial buffer
 // (the _part entry, no waiting, no counter), consecutive grids overlapping
@@ -1446,7 +1467,9 @@ int launch_batched(mf_kernel* k, uint32_t count, const void* const* data, const 
   mf_context* c = k->ctx;
   int maxgrid = 1;
   for (uint32_t i = 0; i < count; i++) maxgrid = std::max(maxgrid, grid_for(k, ns[i]));
-  const uint32_t chunk = std::min(count, kChunk);
+  // evaluations too small to fill the device: many to a launch
+  const bool batch = batch_fits(k, maxgrid);
+  const uint32_t chunk = std::min(count, batch ? uint32_t(k->lowered.batch_max) : kChunk);
   const uint64_t pstride = uint64_t(maxgrid) * k->n_outputs;  // float2 per evaluation
   if (c->ring_cap < chunk * pstride) {
     if (c->ring) {
@@ -1467,7 +1490,8 @@ int launch_batched(mf_kernel* k, uint32_t count, const void* const* data, const 
     c->ring_grids_cap = kChunk;
   }
   const size_t ab = k->lowered.args_bytes();
-  std::vector<unsigned char> pv(ab, 0);
+  const size_t jb = sizeof(BatchJob) + ab;  // mf_job
+  std::vector<unsigned char> pv(batch ? jb * size_t(k->lowered.batch_max) : ab, 0);
   std::vector<unsigned> grids(chunk);
   unsigned* status = c->status;
   for (uint32_t first = 0; first < count; first += chunk) {
@@ -1475,6 +1499,17 @@ int launch_batched(mf_kernel* k, uint32_t count, const void* const* data, const 
     for (uint32_t i = 0; i < m; i++) {
       const uint32_t e = first + i;
       grids[i] = unsigned(grid_for(k, ns[e]));
+      if (batch) {
+        unsigned char* job = pv.data() + jb * i;
+        const BatchJob b{data[e], strides[e], ns[e], grids[i]};
+        std::memcpy(job, &b, sizeof b);
+        try {
+          k->lowered.fill_args(params + uint64_t(e) * k->n_params, k->n_params, job + sizeof b);
+        } catch (const std::exception& ex) {
+          return fail(MF_ERR_INVALID, std::string("parameter evaluation: ") + ex.what());
+        }
+        continue;
+      }
       try {
         k->lowered.fill_args(params + uint64_t(e) * k->n_params, k->n_params, pv.data());
       } catch (const std::exception& ex) {
@@ -1496,6 +1531,20 @@ int launch_batched(mf_kernel* k, uint32_t count, const void* const* data, const 
       cfg.numAttrs = i > 0 ? 1 : 0;
       res_yield(k->ctx);
       MF_CUDA_TRY(cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(k->fn_part), args));
+    }
+    if (batch) {
+      float2* ring = c->ring;
+      uint64_t ps = pstride;
+      // about four rounds of blocks on the device, at most kBatchGroup evaluations a block
+      const uint64_t want = uint64_t(c->num_sms) * uint64_t(k->blocks_per_sm) * 4;
+      uint32_t group = uint32_t(std::max<uint64_t>(
+          1, std::min<uint64_t>(mf::kBatchGroup, uint64_t(m) * uint64_t(maxgrid) / want)));
+      uint32_t mm = m;
+      void* args[] = {pv.data(), &ring, &ps, &mm, &group};
+      res_yield(k->ctx);
+      MF_CUDA_TRY(cudaLaunchKernel(reinterpret_cast<const void*>(k->fn_batch),
+                                   dim3(unsigned(maxgrid), (m + group - 1) / group), dim3(k->lowered.block), args, 0,
+                                   c->stream));
     }
     // the chunk's grid sizes: one value when they are all equal (evaluations
     // of one size, the common case), else a copy (pageable source: staged
