@@ -58,10 +58,23 @@ namespace {
   } while (0)
 
 // ------------------------------------------------------------ compile cache --
+struct LoadedModule;
 struct CompiledImage {
   std::vector<char> cubin;
   int regs = -1, spill = -1;
   std::string log;
+  std::weak_ptr<LoadedModule> loaded;  // under g_cache_mu
+};
+
+// An image's code on the device, shared by the kernels built from it and
+// unloaded with the last of them. Several datasets of one model (a kernel
+// each) then run the same code: alternating between three copies of the Crystal
+// Ball kernel's fetched it anew every call.
+struct LoadedModule {
+  cudaLibrary_t lib = nullptr;
+  ~LoadedModule() {
+    if (lib) cudaLibraryUnload(lib);
+  }
 };
 
 std::mutex g_cache_mu;
@@ -177,6 +190,17 @@ int compile_source(const std::string& src, const std::string& name, std::shared_
   return MF_OK;
 }
 
+int load_image(const std::shared_ptr<CompiledImage>& img, std::shared_ptr<LoadedModule>& out) {
+  std::lock_guard<std::mutex> lk(g_cache_mu);
+  out = img->loaded.lock();
+  if (out) return MF_OK;
+  auto m = std::make_shared<LoadedModule>();
+  MF_CUDA_TRY(cudaLibraryLoadData(&m->lib, img->cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0));
+  img->loaded = m;
+  out = m;
+  return MF_OK;
+}
+
 }  // namespace
 
 // ----------------------------------------------------------------- objects --
@@ -289,7 +313,7 @@ struct mf_kernel {
   uint32_t n_inputs = 0, n_params = 0, n_outputs = 0, n_gen_dims = 0;
   mf::LoweredKernel lowered;
   std::shared_ptr<CompiledImage> image;
-  cudaLibrary_t lib = nullptr;
+  std::shared_ptr<LoadedModule> module;
   cudaKernel_t fn = nullptr;
   cudaKernel_t fn_seg = nullptr;
   cudaKernel_t fn_prep = nullptr;  // REDUCE kernels reading prepared columns
@@ -909,19 +933,20 @@ int mf_kernel_build(mf_context* c, const mf_kernel_desc* d, mf_kernel** out) {
   int rc = compile_source(k->lowered.source, k->name, k->image, k->lowered.entry);
   if (rc) return rc;
   MF_CUDA_TRY(cudaSetDevice(c->device));
-  MF_CUDA_TRY(cudaLibraryLoadData(&k->lib, k->image->cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0));
-  MF_CUDA_TRY(cudaLibraryGetKernel(&k->fn, k->lib, k->lowered.entry.c_str()));
+  rc = load_image(k->image, k->module);
+  if (rc) return rc;
+  MF_CUDA_TRY(cudaLibraryGetKernel(&k->fn, k->module->lib, k->lowered.entry.c_str()));
   if (d->kind == MF_KERNEL_REDUCE || d->kind == MF_KERNEL_GENERATE)
-    MF_CUDA_TRY(cudaLibraryGetKernel(&k->fn_seg, k->lib, (k->lowered.entry + "_segments").c_str()));
+    MF_CUDA_TRY(cudaLibraryGetKernel(&k->fn_seg, k->module->lib, (k->lowered.entry + "_segments").c_str()));
   if (d->kind == MF_KERNEL_REDUCE) {
-    MF_CUDA_TRY(cudaLibraryGetKernel(&k->fn_part, k->lib, (k->lowered.entry + "_part").c_str()));
+    MF_CUDA_TRY(cudaLibraryGetKernel(&k->fn_part, k->module->lib, (k->lowered.entry + "_part").c_str()));
     if (k->lowered.batch_max)
-      MF_CUDA_TRY(cudaLibraryGetKernel(&k->fn_batch, k->lib, (k->lowered.entry + "_batch").c_str()));
-    MF_CUDA_TRY(cudaLibraryGetKernel(&k->fn_combine, k->lib, (k->lowered.entry + "_combine").c_str()));
-    MF_CUDA_TRY(cudaLibraryGetKernel(&k->fn_multi, k->lib, (k->lowered.entry + "_multi").c_str()));
+      MF_CUDA_TRY(cudaLibraryGetKernel(&k->fn_batch, k->module->lib, (k->lowered.entry + "_batch").c_str()));
+    MF_CUDA_TRY(cudaLibraryGetKernel(&k->fn_combine, k->module->lib, (k->lowered.entry + "_combine").c_str()));
+    MF_CUDA_TRY(cudaLibraryGetKernel(&k->fn_multi, k->module->lib, (k->lowered.entry + "_multi").c_str()));
   }
   if (k->lowered.prep) {
-    MF_CUDA_TRY(cudaLibraryGetKernel(&k->fn_prep, k->lib, (k->lowered.entry + "_prep").c_str()));
+    MF_CUDA_TRY(cudaLibraryGetKernel(&k->fn_prep, k->module->lib, (k->lowered.entry + "_prep").c_str()));
     k->prep_key = prep_key(k.get());
   }
   if (k->lowered.smem_bytes > 48 * 1024) {
@@ -1346,10 +1371,10 @@ int mf_kernel_free(mf_kernel* k) {
   if (k->f64) mf_kernel_free(k->f64);
   mf_context* c = k->ctx;
   res_forget(k);
-  if (k->lib) {
+  if (k->module) {
     cudaSetDevice(c->device);
-    cudaStreamSynchronize(c->stream);
-    cudaLibraryUnload(k->lib);
+    cudaStreamSynchronize(c->stream);  // its launches are done; the last kernel of the image unloads it
+    k->module.reset();
   }
   const bool counted = k->holds_ref;
   delete k;
