@@ -9,7 +9,8 @@ from morefit_gb300.backend import lower_source
 
 
 def _part(src):
-    return src[src.index("mf_reduce_part("):src.index("_combine(")]
+    i = src.index("mf_reduce_part(")
+    return src[i:src.index('extern "C"', i)]
 
 
 def test_exchanged_operands_and_powers_share():
@@ -58,4 +59,33 @@ def test_shared_values_equal_their_own_kernels():
         for j, e in enumerate(exprs[:4]):
             assert np.array_equal(got[finite, j], values([e], n, m)[finite, 0]), (e, n, m)
         assert (np.abs(got[finite, 4] - ref[finite, 4]) <= 3e-14 * ref[finite, 4]).all()
+    b.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 255, 513, 5003])
+def test_sums_of_products_match_fp64(n):
+    """Sums and differences of products and values, nested and negated, as an
+    output of their own, under a logarithm, plus a parameter-only value, and
+    used by two outputs: within 1e-12 of the sum of the terms' magnitudes."""
+    from morefit_gb300.backend import CUDABackend, CUDABlock
+    b = CUDABackend(0, resident_idle_us=0)
+    rng = np.random.default_rng(n)
+    x, y = rng.uniform(0.5, 1.5, n), rng.uniform(-1.0, 1.0, n)
+    a, c = 0.37, -1.25
+    s = "((x*y)+-(((y*y)*a))+x+-((c*y)))"
+    exprs = ["((x*y)+-((y*y*x))+(x+-(y)))", f"log((7.0+{s}))", "((x*y)+-((y*x*x))+a)", f"({s}*y)", f"({s}+(x*x*x))",
+             "-((-((x*x))+-(y)))", "((x+y)+(x*a)+(y*c)+1.5)"]
+    blk = CUDABlock(b, np.float64)
+    blk.MakeComputeKernel("sums", 0, ["x", "y"], ["r"] * len(exprs), ["a", "c"], exprs, True)
+    blk.CopyToInputBuffer(np.stack([x, y]))
+    blk.CopyToParameterBuffer([a, c])
+    blk.SubmitKernel()
+    S = x * y - y * y * a + x - c * y
+    ref = np.stack([x * y - y * y * x + (x - y), np.log(7.0 + S), x * y - y * x * x + a, S * y, S + x * x * x, x * x + y,
+                    x + y + x * a + y * c + 1.5])
+    got = blk.CopyFromKahanBuffer()
+    assert (np.abs(got - ref.sum(axis=1)) <= 1e-12 * np.maximum(np.abs(ref).sum(axis=1), 1.0)).all()
+    seg = blk.SubmitSegments([0], [n], [[a, c]])[0]
+    assert (np.abs(seg - ref.sum(axis=1)) <= 1e-12 * np.maximum(np.abs(ref).sum(axis=1), 1.0)).all()
     b.close()
