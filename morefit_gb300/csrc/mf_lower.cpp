@@ -1503,6 +1503,10 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
     // normalisation terms of Hessian outputs): x is accumulated and the
     // thread's event count times u added once, before the block reduction.
     std::vector<int> addu(roots.size(), -1), addsign(roots.size(), 0), accnode(roots);
+    // Double-float outputs x * u with u parameter-only: x is accumulated and
+    // multiplied by u once (the S+P-wave Hessian scales 36 of its 105 outputs
+    // by (1 - FS): a product per event and output less).
+    std::vector<std::vector<int>> scale(roots.size());
     // FP32 REDUCE bodies (mixed precision) whose only output is the logarithm
     // of a dot product of per-event values with parameter-only factors (the
     // fitter's NLL kernel for a density linear in its prepared columns): that
@@ -1625,10 +1629,25 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
           }
           continue;
         }
-        if (n.op == Op::Mul && !n.uniform && uses[r] == 1 && !chains.count(r) && !skip[r]) {
-          fused[j] = {n.a, n.b};
-          skip[r] = 1;
-        }
+        // what output j accumulates of node x: parameter-only factors aside, a
+        // product multiplied straight into the accumulator
+        auto accumulate = [&](int x) {
+          auto product = [&](int k) {
+            return ns[k].op == Op::Mul && !ns[k].uniform && uses[k] == 1 && !chains.count(k) && !skip[k];
+          };
+          while (product(x) && ns[ns[x].a].uniform != ns[ns[x].b].uniform) {
+            const bool first = ns[ns[x].a].uniform;
+            scale[j].push_back(first ? ns[x].a : ns[x].b);
+            skip[x] = 1;
+            x = first ? ns[x].b : ns[x].a;
+          }
+          accnode[j] = x;
+          if (product(x)) {
+            fused[j] = {ns[x].a, ns[x].b};
+            skip[x] = 1;
+          }
+        };
+        if (n.op == Op::Mul && !n.uniform && uses[r] == 1 && !chains.count(r) && !skip[r]) accumulate(r);
         if (ar == Ar::DW && !lf && !skip[r] && uses[r] == 1 && !n.uniform && (n.op == Op::Add || n.op == Op::Sub)) {
           int x = -1, u = -1, sg = 0;
           if (ns[n.b].uniform && !ns[n.a].uniform) {
@@ -1643,13 +1662,8 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
           if (x >= 0 && !skip[x]) {
             addu[j] = u;
             addsign[j] = sg;
-            accnode[j] = x;
             skip[r] = 1;
-            const Node& xn = ns[x];
-            if (xn.op == Op::Mul && uses[x] == 1 && !chains.count(x)) {
-              fused[j] = {xn.a, xn.b};
-              skip[x] = 1;
-            }
+            accumulate(x);
           }
         }
         // an output that is the logarithm of a per-event value (plus or minus a
@@ -2074,6 +2088,11 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
     };
     // Per-thread partials of the log-product outputs, before the block reduction.
     auto acc_finish = [&](std::ostringstream& o) {
+      for (int j = 0; j < M; j++) {
+        for (size_t q = 0; q < scale[j].size(); q++)
+          o << "  " << accref(j) << " = mf_dw_mul(" << (q ? "" : "mf_dw_renorm(") << accref(j) << (q ? "" : ")") << ", "
+            << eref(scale[j][q]) << ");\n";
+      }
       for (int j = 0; j < M; j++)
         if (addu[j] >= 0)
           o << "  " << accref(j) << " = " << (addsign[j] > 0 ? "mf_dw_add" : "mf_dw_sub") << "(mf_dw_renorm("

@@ -89,3 +89,30 @@ def test_sums_of_products_match_fp64(n):
     seg = blk.SubmitSegments([0], [n], [[a, c]])[0]
     assert (np.abs(seg - ref.sum(axis=1)) <= 1e-12 * np.maximum(np.abs(ref).sum(axis=1), 1.0)).all()
     b.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 257, 5003])
+def test_outputs_scaled_by_parameters_match_fp64(n):
+    """Outputs with parameter-only factors, which are applied to the sum: a
+    column, a product, a function and a sum times one and two of them, plus a
+    parameter-only value, and one whose factor is zero: within 1e-12 of the sum
+    of the terms' magnitudes."""
+    from morefit_gb300.backend import CUDABackend, CUDABlock
+    b = CUDABackend(0, resident_idle_us=0)
+    rng = np.random.default_rng(n + 7)
+    x, y = rng.uniform(0.5, 1.5, n), rng.uniform(-1.0, 1.0, n)
+    a, c, z = 0.37, -1.25, 0.0
+    exprs = ["(x*a)", "((x*y)*a)", "(a*(c*(x*y)))", "((x*a)+c)", "(c+((x*y*y)*a))", "(sqrt(x)*c)", "(((x*y)+(y*y))*a)",
+             "((x*y)*z)", "(((x*y)+(x*x*y)+y)*(a*c))"]
+    blk = CUDABlock(b, np.float64)
+    blk.MakeComputeKernel("scaled", 0, ["x", "y"], ["r"] * len(exprs), ["a", "c", "z"], exprs, True)
+    blk.CopyToInputBuffer(np.stack([x, y]))
+    blk.CopyToParameterBuffer([a, c, z])
+    blk.SubmitKernel()
+    ref = np.stack([x * a, x * y * a, a * c * x * y, x * a + c, c + x * y * y * a, np.sqrt(x) * c, (x * y + y * y) * a,
+                    0.0 * x, (x * y + x * x * y + y) * a * c])
+    tol = 1e-12 * np.maximum(np.abs(ref).sum(axis=1), 1.0)
+    assert (np.abs(blk.CopyFromKahanBuffer() - ref.sum(axis=1)) <= tol).all()
+    assert (np.abs(blk.SubmitSegments([0], [n], [[a, c, z]])[0] - ref.sum(axis=1)) <= tol).all()
+    b.close()
