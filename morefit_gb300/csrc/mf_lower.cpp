@@ -2716,14 +2716,24 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
     // GENERATE: accept-reject generation, one xoshiro128++ stream per
     // `lanes` threads of a warp (a power of two up to 32, chosen at launch).
     // Stream t owns events [t*nper, min((t+1)*nper, n)) and makes them from
-    // its proposals in order. Lane j of the stream's lanes tests proposals j,
-    // lanes + j, ...: it starts (D+1) * j draws into the stream and skips the
-    // other lanes' (D+1) * (lanes - 1) draws after each of its own (six
-    // logic instructions a draw). The lanes' decisions meet in a ballot, and
-    // the accepted proposals take the stream's next events in the order of
-    // the proposals, so the events are those of one thread walking the
-    // stream, and no lane waits for another stream's next acceptance. Measured
-    // figures: generator_lanes() in mf_runtime.cpp.
+    // its proposals in order. In a turn, lane j of the stream's lanes tests
+    // proposals j*chunk ... (j+1)*chunk - 1 of the next lanes*chunk, and the
+    // accepted ones take the stream's next events in the order of the
+    // proposals, so the events are those of one thread walking the stream,
+    // and no lane waits for another stream's next acceptance.
+    //
+    // What bounds it: instructions, of which a third skipped the other lanes'
+    // draws (six logic instructions a draw, (D+1) * (lanes - 1) draws after
+    // each proposal) while a turn was one proposal a lane. With chunk > 1 a
+    // lane jumps over them by a table of its own fixed number of steps, a
+    // linear map of the 128-bit state: 64 loads and about 200 instructions
+    // for `chunk` proposals and any number of lanes. The table is 8 KB of
+    // shared memory, two words an entry so that the 16 values of a nibble lie
+    // in all 32 banks once (with four words an entry the loads' bank
+    // conflicts took twice the time), and every block makes it for itself.
+    // K*mumu P wave, 1M events: 337 -> 215 us. chunk = 1 keeps the stepping,
+    // for streams too short to pay for the table. Both forms measured, and
+    // where the line lies: generator_shape() in mf_runtime.cpp.
     const int D = int(gen->dims.size());
     s << R"CUDA(__device__ __forceinline__ unsigned mf_rotl(unsigned x, int k) { return (x << k) | (x >> (32 - k)); }
 struct mf_rng { unsigned s0, s1, s2, s3; };
@@ -2735,6 +2745,58 @@ __device__ __forceinline__ unsigned mf_rng_draw(mf_rng& s) {
   const unsigned r = mf_rotl(s.s0 + s.s3, 7) + s.s0;
   mf_rng_step(s);
   return r;
+}
+// A fixed number of steps is a 128 x 128 matrix over GF(2); `tab` holds, for
+// each of the state's 32 nibbles and each value of it, the columns it adds.
+__device__ __forceinline__ mf_rng mf_rng_jump(const uint2 (*tab)[512], const mf_rng s) {
+  unsigned w[4] = {s.s0, s.s1, s.s2, s.s3};
+  mf_rng r = {0u, 0u, 0u, 0u};
+#pragma unroll 1
+  for (int k = 0; k < 4; k++) {
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      const unsigned v = k * 128 + q * 16 + ((w[0] >> (4 * q)) & 15u);
+      const uint2 e = tab[0][v], f = tab[1][v];
+      r.s0 ^= e.x; r.s1 ^= e.y; r.s2 ^= f.x; r.s3 ^= f.y;
+    }
+    w[0] = w[1]; w[1] = w[2]; w[2] = w[3];
+  }
+  return r;
+}
+// Lane `sub` of a stream goes `sub * steps` steps ahead, and `tab` becomes the
+// table of `lanes * steps` steps. Column threadIdx.x of the matrix is stepped
+// from its unit vector; applying a table to its own columns doubles the steps.
+// All threads of a block of MF_BLOCK >= 128 call this together.
+__device__ __forceinline__ mf_rng mf_rng_spread(mf_rng st, unsigned steps, unsigned sub, unsigned lanes, uint4* col,
+                                                uint2 (*tab)[512]) {
+  const unsigned t = threadIdx.x & 127u, bit = 1u << (t & 31u);
+  mf_rng c = {t < 32u ? bit : 0u, (t >> 5) == 1u ? bit : 0u, (t >> 5) == 2u ? bit : 0u, t >= 96u ? bit : 0u};
+  for (unsigned k = 0; k < steps; k++) mf_rng_step(c);
+  for (unsigned b = 1;; b *= 2) {
+    if (threadIdx.x < 128u) col[t] = make_uint4(c.s0, c.s1, c.s2, c.s3);
+    __syncthreads();
+    if (threadIdx.x < 128u) {
+      // four values of nibble t / 4: the upper two bits are those of t
+      const uint4* n = col + (t & ~3u);
+      const uint4 p = n[0], q = n[1], u = n[2], v = n[3];
+      const unsigned mu = (t & 1u) ? MF_FULL : 0u, mv = (t & 2u) ? MF_FULL : 0u;
+      const uint2 z0 = make_uint2((u.x & mu) ^ (v.x & mv), (u.y & mu) ^ (v.y & mv));
+      const uint2 z1 = make_uint2((u.z & mu) ^ (v.z & mv), (u.w & mu) ^ (v.w & mv));
+      uint2 *lo = tab[0] + 4u * t, *hi = tab[1] + 4u * t;
+      lo[0] = z0;
+      lo[1] = make_uint2(z0.x ^ p.x, z0.y ^ p.y);
+      lo[2] = make_uint2(z0.x ^ q.x, z0.y ^ q.y);
+      lo[3] = make_uint2(z0.x ^ p.x ^ q.x, z0.y ^ p.y ^ q.y);
+      hi[0] = z1;
+      hi[1] = make_uint2(z1.x ^ p.z, z1.y ^ p.w);
+      hi[2] = make_uint2(z1.x ^ q.z, z1.y ^ q.w);
+      hi[3] = make_uint2(z1.x ^ p.z ^ q.z, z1.y ^ p.w ^ q.w);
+    }
+    __syncthreads();
+    if (b >= lanes) return st;
+    if (sub & b) st = mf_rng_jump(tab, st);
+    c = mf_rng_jump(tab, c);
+  }
 }
 )CUDA";
     if (!ar32) s << kEfPrelude;
@@ -2857,66 +2919,104 @@ __device__ __forceinline__ unsigned mf_rng_draw(mf_rng& s) {
     }
     // one stream's events, `lanes` threads a stream; from, to, maxprob and
     // the parameter-only values are defined
-    auto accept_reject = [&]() {
-      for (int k : filter_uniform)
-        s << "  const mf_ef uf" << k << " = mf_ef_from(" << em.ref(k, "u") << ");\n";
-      if (filter) s << "  const mf_ef maxprob_f = mf_ef_from(maxprob);\n";
-      s << "  const unsigned sub = threadIdx.x & (lanes - 1u), first = (threadIdx.x & 31u) - sub;\n"
-        << "  const unsigned mine = lanes == 32u ? MF_FULL : ((1u << lanes) - 1u);\n"
-        << "  for (unsigned k = 0; k < sub; k++) {\n#pragma unroll\n    for (int q = 0; q < " << D + 1
-        << "; q++) mf_rng_step(st);\n  }\n"
-        << "  mf_u64 i = from, tried = 0;\n  bool run = i < to;\n"
-        << "  while (__any_sync(MF_FULL, run)) {\n";
-      for (int d = 0; d <= D; d++) s << "    const unsigned d" << d << " = mf_rng_draw(st);\n";
-      s << "    for (unsigned k = 1; k < lanes; k++) {\n#pragma unroll\n      for (int q = 0; q < " << D + 1
-        << "; q++) mf_rng_step(st);\n    }\n"
-        << "    bool acc = false;\n"
-        << "    if (run && tried + sub < max_tries) {\n";
-      auto draw = [](int d) { return "d" + std::to_string(d); };
+    // A chunk's accepted proposals wait in shared memory (at most 24 KB) for
+    // their events' places.
+    const unsigned chunk_max = out.gen_chunk = std::max(1u, std::min(8u, 48u / unsigned(D)));
+    auto draw = [](int d) { return "d" + std::to_string(d); };
+    auto slot = [](int d) { return "outp[(mf_u64)" + std::to_string(d) + " * out_stride + at]"; };
+    // acc = the decision on the proposal with the draws d0...
+    auto decide = [&]() {
+      for (int d = 0; d <= D; d++) s << "      const unsigned d" << d << " = mf_rng_draw(st);\n";
+      s << "      bool acc = false;\n"
+        << "      if (run && tried + at_try < max_tries) {\n";
       if (filter) {
         for (int d = 0; d < D; d++) {
           const double lo = printed15(gen->lo[d]), del = printed15(gen->hi[d] - gen->lo[d]);
           char eb[48];
           std::snprintf(eb, sizeof eb, "%.9ef", (std::fabs(lo) + std::fabs(del)) * 0x1p-22);
-          s << "      const mf_ef xe" << d << " = mf_ef_make(__fmaf_rn(" << fmt_const(del, true) << ", (float)d" << d
+          s << "        const mf_ef xe" << d << " = mf_ef_make(__fmaf_rn(" << fmt_const(del, true) << ", (float)d" << d
             << " * 2.3283064365386963e-10f, " << fmt_const(lo, true) << "), " << eb << ");\n";
         }
-        s << "      bool amb = false;\n      const mf_ef p = " << filter_call << ";\n"
-          << "      const mf_ef ug = mf_ef_mul(maxprob_f, mf_ef_make((float)d" << D
+        s << "        bool amb = false;\n        const mf_ef p = " << filter_call << ";\n"
+          << "        const mf_ef ug = mf_ef_mul(maxprob_f, mf_ef_make((float)d" << D
           << " * 2.3283064365386963e-10f, 0x1p-24f));\n"
-          << "      const float gap = __fsub_rn(p.v, ug.v);\n"
-          << "      acc = gap > 0.0f;\n"
-          << "      if (amb || !(fabsf(gap) > 1.01f * (p.e + ug.e) + 0x1p-23f * fabsf(gap))) {  // in FP64\n";
-        for (int d = 0; d < D; d++) s << "        const double x" << d << " = " << coordinate(d, draw(d)) << ";\n";
-        emit_body(s, "        ");
-        s << "        acc = __dmul_rn(maxprob, d" << D << " * 2.3283064365386963e-10) < r0;\n      }\n";
+          << "        const float gap = __fsub_rn(p.v, ug.v);\n"
+          << "        acc = gap > 0.0f;\n"
+          << "        if (amb || !(fabsf(gap) > 1.01f * (p.e + ug.e) + 0x1p-23f * fabsf(gap))) {  // in FP64\n";
+        for (int d = 0; d < D; d++) s << "          const double x" << d << " = " << coordinate(d, draw(d)) << ";\n";
+        emit_body(s, "          ");
+        s << "          acc = __dmul_rn(maxprob, d" << D << " * 2.3283064365386963e-10) < r0;\n        }\n";
       } else {
-        for (int d = 0; d < D; d++) s << "      const float x" << d << " = " << coordinate(d, draw(d)) << ";\n";
-        emit_body(s, "      ");
-        s << "      acc = __fmul_rn(maxprob, (float)d" << D << " * 2.3283064365386963e-10f) < r0;\n";
+        for (int d = 0; d < D; d++) s << "        const float x" << d << " = " << coordinate(d, draw(d)) << ";\n";
+        emit_body(s, "        ");
+        s << "        acc = __fmul_rn(maxprob, (float)d" << D << " * 2.3283064365386963e-10f) < r0;\n";
       }
-      s << "    }\n"
-        << "    const unsigned m = (__ballot_sync(MF_FULL, acc) >> first) & mine;\n"
-        << "    if (acc) {\n      const mf_u64 at = i + __popc(m & ((1u << sub) - 1u));\n      if (at < to) {\n";
-      for (int d = 0; d < D; d++) {
-        const std::string slot = "outp[(mf_u64)" + std::to_string(d) + " * out_stride + at]";
-        if (filter)
-          s << "        " << slot << " = __longlong_as_double((long long)d" << d << ");\n";
-        else
-          s << "        " << slot << " = " << coordinate(d, draw(d)) << ";\n";
+      s << "      }\n";
+    };
+    auto keep_event = [&](const std::string& pad, const std::function<std::string(int)>& w) {
+      for (int d = 0; d < D; d++)
+        s << pad << slot(d) << " = "
+          << (filter ? "__longlong_as_double((long long)" + w(d) + ")" : coordinate(d, w(d))) << ";\n";
+    };
+    auto end_of_turn = [&]() {
+      s << "      if (run && i >= to) {\n        run = false;\n      } else if (run && tried >= max_tries) {\n"
+        << "        run = false;\n        if (sub == 0u) atomicOr(status, 1u);\n      }\n    }\n";
+    };
+    auto accept_reject = [&]() {
+      if (chunk_max > 1)
+        s << "  __shared__ uint4 mf_col[MF_BLOCK];\n  __shared__ uint2 mf_tab[2][512];\n  __shared__ unsigned mf_kept["
+          << chunk_max * D << " * MF_BLOCK];\n";
+      for (int k : filter_uniform)
+        s << "  const mf_ef uf" << k << " = mf_ef_from(" << em.ref(k, "u") << ");\n";
+      if (filter) s << "  const mf_ef maxprob_f = mf_ef_from(maxprob);\n";
+      s << "  const unsigned sub = threadIdx.x & (lanes - 1u);\n"
+        << "  mf_u64 i = from, tried = 0;\n  bool run = i < to;\n";
+      if (chunk_max > 1) {
+        s << "  if (chunk > 1u) {\n    st = mf_rng_spread(st, chunk * " << D + 1 << "u, sub, lanes, mf_col, mf_tab);\n"
+          << "    while (__any_sync(MF_FULL, run)) {\n      mf_col[threadIdx.x] = make_uint4(st.s0, st.s1, st.s2, st.s3);\n"
+          << "      unsigned c = 0;\n#pragma unroll 1\n"
+          << "      for (unsigned q = 0; q < chunk; q++) {\n      const unsigned at_try = sub * chunk + q;\n";
+        decide();
+        s << "      if (acc) {\n";
+        const std::string KD = " * " + std::to_string(D) + "u + ";
+        for (int d = 0; d < D; d++)
+          s << "        mf_kept[(c" << KD << d << "u) * MF_BLOCK + threadIdx.x] = d" << d << ";\n";
+        s << "        c++;\n      }\n      }\n      const uint4 w = mf_col[threadIdx.x];\n"
+          << "      st = mf_rng_jump(mf_tab, mf_rng{w.x, w.y, w.z, w.w});\n"
+          << "      unsigned upto = c;  // events of this and the stream's earlier lanes\n"
+          << "      for (unsigned o = 1; o < lanes; o *= 2) {\n"
+          << "        const unsigned v = __shfl_up_sync(MF_FULL, upto, o, lanes);\n        if (sub >= o) upto += v;\n"
+          << "      }\n      for (unsigned j = 0; j < c; j++) {\n        const mf_u64 at = i + (upto - c) + j;\n"
+          << "        if (at < to) {\n";
+        keep_event("          ", [&](int d) {
+          return "mf_kept[(j" + KD + std::to_string(d) + "u) * MF_BLOCK + threadIdx.x]";
+        });
+        s << "        }\n      }\n      i += __shfl_sync(MF_FULL, upto, lanes - 1u, lanes);\n      tried += lanes * chunk;\n";
+        end_of_turn();
+        s << "  } else {\n";
+      } else {
+        s << "  {\n";
       }
-      s << "      }\n    }\n"
-        << "    i += __popc(m);\n    tried += lanes;\n"
-        << "    if (run && i >= to) {\n      run = false;\n    } else if (run && tried >= max_tries) {\n"
-        << "      run = false;\n      if (sub == 0u) atomicOr(status, 1u);\n    }\n  }\n";
+      s << "    const unsigned first = (threadIdx.x & 31u) - sub;\n"
+        << "    const unsigned mine = lanes == 32u ? MF_FULL : ((1u << lanes) - 1u);\n"
+        << "    for (unsigned k = 0; k < sub; k++) {\n#pragma unroll\n      for (int q = 0; q < " << D + 1
+        << "; q++) mf_rng_step(st);\n    }\n"
+        << "    while (__any_sync(MF_FULL, run)) {\n      const unsigned at_try = sub;\n";
+      decide();
+      s << "      for (unsigned k = 1; k < lanes; k++) {\n#pragma unroll\n        for (int q = 0; q < " << D + 1
+        << "; q++) mf_rng_step(st);\n      }\n"
+        << "      const unsigned m = (__ballot_sync(MF_FULL, acc) >> first) & mine;\n"
+        << "      if (acc) {\n        const mf_u64 at = i + __popc(m & ((1u << sub) - 1u));\n        if (at < to) {\n";
+      keep_event("          ", draw);
+      s << "        }\n      }\n      i += __popc(m);\n      tried += lanes;\n";
+      end_of_turn();
+      s << "  }\n";
       if (filter) {
         s << "  // the stored draws become coordinates\n  __syncwarp();\n  if (i > to) i = to;\n"
           << "  for (mf_u64 at = from + sub; at < i; at += lanes) {\n";
-        for (int d = 0; d < D; d++) {
-          const std::string slot = "outp[(mf_u64)" + std::to_string(d) + " * out_stride + at]";
-          s << "    { const unsigned w = (unsigned)__double_as_longlong(" << slot << ");\n      " << slot << " = "
+        for (int d = 0; d < D; d++)
+          s << "    { const unsigned w = (unsigned)__double_as_longlong(" << slot(d) << ");\n      " << slot(d) << " = "
             << coordinate(d, "w") << "; }\n";
-        }
         s << "  }\n";
       }
       s << "}\n";
@@ -2924,7 +3024,7 @@ __device__ __forceinline__ unsigned mf_rng_draw(mf_rng& s) {
     s << "extern \"C\" __global__ void __launch_bounds__(MF_BLOCK) " << out.entry
       << "(const unsigned* __restrict__ seeds, unsigned nseeds, mf_u64 n, mf_u64 nper, mf_par P, " << ST
       << "* __restrict__ outp, mf_u64 out_stride, unsigned* __restrict__ status, unsigned long long max_tries,"
-      << " unsigned long long splitmix_seed, unsigned lanes) {\n";
+      << " unsigned long long splitmix_seed, unsigned lanes, unsigned chunk) {\n";
     // whole warps stay in the loop: threads beyond the last stream have no events
     s << "  const mf_u64 thread = (mf_u64)blockIdx.x * MF_BLOCK + threadIdx.x;\n"
       << "  const bool have = thread / lanes < nseeds;\n"
@@ -2956,7 +3056,7 @@ __device__ __forceinline__ unsigned mf_rng_draw(mf_rng& s) {
       << " const mf_u64* __restrict__ seg_begin, const unsigned* __restrict__ seg_count,"
       << " const mf_par* __restrict__ seg_params, const double* __restrict__ seg_maxprob, " << ST
       << "* __restrict__ outp, mf_u64 out_stride, unsigned* __restrict__ status, unsigned long long max_tries,"
-      << " unsigned lanes) {\n";
+      << " unsigned lanes, unsigned chunk) {\n";
     s << "  const mf_u64 thread = (mf_u64)blockIdx.x * MF_BLOCK + threadIdx.x;\n"
       << "  const bool have = thread / lanes < nthreads;\n"
       << "  const unsigned t = have ? (unsigned)(thread / lanes) : 0u;\n"

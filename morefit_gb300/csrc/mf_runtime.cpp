@@ -2476,25 +2476,31 @@ int mf_kernel_store_async(mf_kernel* k, const mf_buffer* in, uint64_t in_stride,
   return kernel_store(k, in, in_stride, n, params, n_params, out, out_stride, false);
 }
 
-// Threads per stream of a GENERATE launch (see the generator in mf_lower.cpp):
-// enough that the streams fill the device with about 11 warps per SM, and at
-// least four. With one thread a stream a warp waits for the slowest of its 32
-// streams; every doubling halves that and the serial chain of a stream, and
-// costs one more pass of generator steps per proposal. FP64, one launch and
-// its wait on GB300 (before: one thread a stream, waiting for the warp's
-// slowest lane at every event, double-float density):
-//   threads per stream              1     4     8    16    32   before
-//   K*mumu P wave, 1M events      1127   379   337   373   532   4180 us
-//   S+P wave, 1M                   724   263   236   236   306
-//   mass, 1M                       239   106    96   103   148
-//   P wave, 50k (7143 streams)     153    69    56    58    72
-//   P wave, 1k (1000 streams)       68    37    31    29    28
-//   4096 toys, 65536 streams      3157  2757  2967  3559  4906 (with their tables)
-static unsigned generator_lanes(const mf_context* c, uint64_t streams) {
-  const uint64_t want = uint64_t(c->num_sms) * 352;
-  unsigned lanes = 4;
-  while (lanes < 32 && streams * lanes < want) lanes *= 2;
-  return lanes;
+// Threads per stream of a GENERATE launch and the proposals each tests in a
+// row (see the generator in mf_lower.cpp), for streams of `events` events.
+// Short streams take one proposal a thread and turn: lanes so that the streams
+// fill the device with about 11 warps per SM, and at least four; every
+// doubling halves a stream's serial chain and costs one more pass of generator
+// steps per proposal. Streams of at least 24 events pay for the jump tables
+// (about 10 us a launch) and take the longest chunk: a jump costs the same for
+// any number of lanes, so there are at least 8 lanes, and 16 where a stream
+// has 48 events or more (its last turn tests up to lanes x chunk proposals too
+// many), and 32 where the streams are few. FP64, one launch and its wait on
+// GB300, lanes x chunk as chosen here against the best one-proposal form:
+//   events (streams x events)      P wave      mass      CB + poly   S+P wave
+//   1,000 (1000 x 1)               28          23        24          27
+//   50,000 (7143 x 7)              60          35        41          48
+//   250,000 (8065 x 31)            106 (133)   50 (51)   69 (67)     96 (91)
+//   500,000 (8065 x 62)            139 (201)   65 (66)   87 (92)     133 (139)
+//   1,000,000 (8131 x 123)         215 (351)   81 (95)   121 (143)   194 (242)
+//   1000 toys (16000 x 125)        874 (1065), 4096 toys (65536 x 125) 2440
+//   (2805) with their tables
+static void generator_shape(const mf_context* c, uint64_t streams, uint64_t events, unsigned chunk_max,
+                            unsigned& lanes, unsigned& chunk) {
+  const uint64_t warps11 = uint64_t(c->num_sms) * 352;
+  chunk = events >= 24 ? chunk_max : 1u;
+  lanes = chunk == 1u ? 4 : events >= 48 ? 16 : 8;
+  while (lanes < 32 && streams * lanes < (chunk == 1u ? warps11 : warps11 / 2)) lanes *= 2;
 }
 
 // seeds null: every stream seeded on the device from `splitmix_seed` (the
@@ -2527,8 +2533,9 @@ static int kernel_generate(mf_kernel* k, const uint32_t* seeds, uint32_t nseeds,
   unsigned* status = c->status;
   unsigned long long mt = max_tries ? max_tries : 1000000000ULL;
   unsigned long long sms = splitmix_seed;
-  unsigned lanes = generator_lanes(c, nseeds);
-  void* args[] = {&sd, &nseeds, &n, &nper, pv.data(), &outp, &out_stride, &status, &mt, &sms, &lanes};
+  unsigned lanes, chunk;
+  generator_shape(c, nseeds, nper, k->lowered.gen_chunk, lanes, chunk);
+  void* args[] = {&sd, &nseeds, &n, &nper, pv.data(), &outp, &out_stride, &status, &mt, &sms, &lanes, &chunk};
   const unsigned grid = unsigned((uint64_t(nseeds) * lanes + k->lowered.block - 1) / k->lowered.block);
   res_yield(k->ctx);
   MF_CUDA_TRY(cudaLaunchKernel(reinterpret_cast<const void*>(k->fn), dim3(grid), dim3(k->lowered.block), args, 0,
@@ -2604,9 +2611,12 @@ int mf_kernel_generate_segments(mf_kernel* k, const uint32_t* seeds, uint32_t nt
   void* outp = out->ptr;
   unsigned* status = c->status;
   unsigned long long mt = max_tries ? max_tries : 1000000000ULL;
-  unsigned lanes = generator_lanes(c, nthreads);
+  uint64_t events = 0;
+  for (uint32_t q = 0; q < nseg; q++) events += seg_count[q];
+  unsigned lanes, chunk;
+  generator_shape(c, nthreads, events / nthreads, k->lowered.gen_chunk, lanes, chunk);
   void* args[] = {&d_seeds, &nthreads, &threads_per_seg, &d_begin, &d_count, const_cast<void**>(&d_par), &d_max,
-                  &outp, &out_stride, &status, &mt, &lanes};
+                  &outp, &out_stride, &status, &mt, &lanes, &chunk};
   const unsigned grid = unsigned((uint64_t(nthreads) * lanes + k->lowered.block - 1) / k->lowered.block);
   res_yield(k->ctx);
   MF_CUDA_TRY(cudaLaunchKernel(reinterpret_cast<const void*>(k->fn_seg), dim3(grid), dim3(k->lowered.block), args, 0,

@@ -179,3 +179,74 @@ def test_max_tries_counts_proposals():
         need = max(need, tries)
     assert limit == need and len(fails) == need - 20
     b.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("elem", [np.float64, np.float32], ids=["f64", "f32"])
+@pytest.mark.parametrize("dims,nper,streams", [(1, 23, 3), (1, 24, 3), (2, 47, 5), (7, 48, 3), (24, 30, 2), (25, 30, 2),
+                                               (2, 24, 3400), (1, 48, 1700)])
+def test_runs_of_proposals_equal_the_streams(dims, nper, streams, elem):
+    """Several proposals a thread and turn (8, 6 and 2 of them, in 8, 16 and 32
+    lanes) and the lengths around the rule: the events of one thread walking
+    each stream, here in Python, and the smallest proposal limit that succeeds
+    is the longest walk."""
+    from morefit_gb300._lib import MFError
+    from morefit_gb300.backend import CUDABackend, CUDABlock
+    from morefit_gb300.workloads import seed_rows
+    n = streams * nper - 1
+    seeds = seed_rows(streams, 77)
+    s = [seeds[k].astype(np.uint64) for k in range(4)]
+    m32 = np.uint64(0xFFFFFFFF)
+    rotl = lambda x, k: ((x << np.uint64(k)) | (x >> np.uint64(32 - k))) & m32  # noqa: E731
+
+    def draw():
+        r = (rotl((s[0] + s[3]) & m32, 7) + s[0]) & m32
+        w = (s[1] << np.uint64(9)) & m32
+        s[2] ^= s[0]
+        s[3] ^= s[1]
+        s[1] ^= s[2]
+        s[0] ^= s[3]
+        s[2] ^= w
+        s[3] = rotl(s[3], 11)
+        return r.astype(elem) * elem(2.0**-32)
+    want = np.zeros((dims, n), elem)
+    got = np.zeros(streams, np.int64)
+    quota = np.minimum(nper, n - nper * np.arange(streams))
+    tries = 0
+    while (got < quota).any():
+        x = np.array([draw() for _ in range(dims)])
+        # the density x0 * x_last is exact enough in either type that no
+        # decision of these streams is a tie
+        take = (draw() < x[0] * x[-1]) & (got < quota)
+        at = nper * np.arange(streams) + got
+        want[:, at[take]] = x[:, take]
+        got += take
+        tries += 1
+    names = [f"x{d}" for d in range(dims)]
+    b = CUDABackend(0)
+    blk = CUDABlock(b, elem)
+    blk.MakeGenerateKernel("g", n, [], names, [], [f"(x0*{names[-1]})"], 1.0, ranges=[(0.0, 1.0)] * dims)
+    blk.CopyToSeedBuffer(seeds)
+    blk.SetNevents(n)
+    blk.SubmitKernel(nper=nper, max_tries=tries)
+    assert np.array_equal(blk.output.download(), want)
+    with pytest.raises(MFError):
+        blk.SubmitKernel(nper=nper, max_tries=tries - 1)
+    blk.SubmitKernel(nper=nper)
+    assert np.array_equal(blk.output.download(), want)
+    b.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("workload,n,streams", [("mass", 200003, 8192), ("pwave", 400009, 8192), ("pwave", 6001, 64)])
+def test_long_streams_equal_the_streams(workload, n, streams):
+    """The models' densities at 8, 16 and 32 lanes of 8 proposals."""
+    from morefit_gb300.backend import CUDABackend
+    from morefit_gb300.workloads import generate_events, generate_partition
+    from oracle import mforacle
+    b = CUDABackend(0)
+    cols = generate_events(b, load_spec(workload), n, seed=mforacle.SEED, max_workitems=streams)
+    nper, nseeds = generate_partition(n, streams)
+    assert nper >= 24
+    assert np.array_equal(cols.download(), mforacle.generate_partitioned(workload, n, nper, nseeds))
+    b.close()
