@@ -2298,6 +2298,8 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
     const std::string DT = pair ? "float2" : ST;  // element type the REDUCE entries read
     const std::string XT = ar == Ar::F32 ? "float" : (ar == Ar::F64 || ar == Ar::F32S) ? "double" : "mf_dw";
 
+    s << "__device__ __forceinline__ void mf_prefetch_l2(const void* p) {\n"
+      << "  asm volatile(\"prefetch.global.L2 [%0];\" ::\"l\"(p));\n}\n";
     s << "struct mf_args { double d[" << out.nd << "]; float f[" << out.nf << "]; };\n";
     s << kCombine;
     const int NC = int(out.used_inputs.size());
@@ -2401,6 +2403,12 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
         for (int k : out.used_inputs) s << "    const " << VT << " l" << k << " = c" << k << ";\n";
         for (int k : out.used_inputs)
           s << "    c" << k << " = ahead < n ? " << load_at(k, "ahead") << " : " << VT << "();\n";
+        if (M > 16) {  // the events after those on their way into L2
+          s << "    if (ahead + step < n) {\n";
+          for (int k : out.used_inputs)
+            s << "      mf_prefetch_l2(data + (mf_u64)" << k << " * stride + ahead + step);\n";
+          s << "    }\n";
+        }
         emit_events(s, "    ", "base", nullptr);
         s << "  }\n";
       } else {
@@ -2428,6 +2436,11 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
     // bit, follows the loop's form. Batched evaluations overlap their
     // neighbours instead and keep the registers (P-wave gradient, 64 points of
     // 100k events: 175 without, 190 with).
+    // Of more than 16 outputs (one event per thread and turn, eight warps per
+    // SM) a turn is still shorter than a loaded memory's latency: the events
+    // after the next are asked for in L2 (P-wave Hessian, 1M events 45.3 ->
+    // 42.4 us, 3M 100 -> 93.8; a ring of three turns in shared memory, 42.7;
+    // the gradients, 16 warps per SM and more, lose 3 us by either).
     const bool lone_prefetch = !out.pipelined && NC > 0 && ar == Ar::DW && M <= kAccRegMax;
     auto replace_all = [](std::string& t, const std::string& from, const std::string& to) {
       for (size_t p = t.find(from); p != std::string::npos; p = t.find(from, p + to.size())) t.replace(p, from.size(), to);

@@ -75,3 +75,23 @@ def test_datasets_of_several_sizes():
         for q, i in enumerate(use):
             assert np.array_equal(got[q], likes[i].sums("lh_grad_kernel", th[q])), (q, sizes[i] if i < 10 else "large")
     b.close()
+
+
+@pytest.mark.parametrize("turns,off", [(1, 0), (1, 1), (2, -1), (2, 0), (2, 1), (3, 0), (3, 1)])
+def test_prefetching_loop_reads_the_same_events(turns, off):
+    """A lone Hessian, whose loop loads one turn of the grid ahead and asks for
+    another in L2, against the batched entry's plain loop, at events around
+    whole turns: the same sums bit for bit."""
+    from morefit_gb300.backend import CUDABackend
+    from morefit_gb300.workloads import Likelihood, generate_events, load_spec
+    import torch
+    b = CUDABackend(0, resident_idle_us=0)
+    n = turns * 256 * torch.cuda.get_device_properties(0).multi_processor_count + off
+    like = Likelihood(b, load_spec("pwave"))
+    cols = generate_events(b, load_spec("pwave"), n, seed=3)
+    like.set_device_data(cols)
+    theta = np.array(load_spec("pwave")["truth"])
+    lone = like.sums("lh_hessian_kernel", theta)
+    many = like.sums_many("lh_hessian_kernel", np.stack([theta, theta]))
+    assert np.array_equal(many[0], lone) and np.array_equal(many[1], lone)
+    b.close()
