@@ -2327,13 +2327,42 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
         s << ind << "}\n";
       }
     };
+    // y = one event's value of a prepared column, from the columns src(k) it folds
+    auto emit_fold = [&](std::ostringstream& s, const std::string& ind, const std::string& y, const auto& terms,
+                         const std::function<std::string(int)>& src) {
+      s << ind << "double " << y << " = " << src(terms[0].first) << ";\n";
+      for (size_t t = 1; t < terms.size(); t++) {
+        const double c = terms[t].second;
+        if (c == 1.0)
+          s << ind << y << " = __dadd_rn(" << y << ", " << src(terms[t].first) << ");\n";
+        else if (c == -1.0)
+          s << ind << y << " = __dsub_rn(" << y << ", " << src(terms[t].first) << ");\n";
+        else
+          s << ind << y << " = __fma_rn(" << fmt_const(c, false) << ", " << src(terms[t].first) << ", " << y << ");\n";
+      }
+    };
     // The per-block work of the single-evaluation and the batched entry: the
     // event loop and the block reduction. `prefetch`: a thread's next events
     // are loaded while it computes its present ones, the first before the
     // tables (the same events in the same order, so the same sums).
-    auto block_work = [&](std::ostringstream& s, const bool prefetch) {
-      s << "  mf_launch_dependents();  // the next evaluation may start its event loop on SMs this grid frees\n";
-      if (prefetch) {
+    // `first`: the dataset's columns, unprepared: every vector of them is
+    // prepared here as the _prep entry does and stored for later evaluations.
+    auto block_work = [&](std::ostringstream& s, const bool prefetch, const bool first = false) {
+      if (!first)
+        s << "  mf_launch_dependents();  // the next evaluation may start its event loop on SMs this grid frees\n";
+      std::set<int> raw_cols;
+      const std::string RT = V == 1 ? "double" : "double2";
+      auto raw_at = [&](int k, const std::string& at) {
+        return "__ldg(reinterpret_cast<const " + RT + "*>(raw + (mf_u64)" + std::to_string(k) + " * stride + " + at + "))";
+      };
+      if (first) {
+        for (const auto& terms : fold.cols)
+          for (const auto& t : terms) raw_cols.insert(t.first);
+        s << "  const mf_u64 step = (mf_u64)gridDim.x * MF_BLOCK * " << V << ";\n"
+          << "  mf_u64 base = ((mf_u64)blockIdx.x * MF_BLOCK + threadIdx.x) * " << V << ";\n";
+        for (int k : raw_cols)
+          s << "  " << RT << " c" << k << " = base < stride ? " << raw_at(k, "base") << " : " << RT << "();\n";
+      } else if (prefetch) {
         s << "  const mf_u64 step = (mf_u64)gridDim.x * MF_BLOCK * " << V << ";\n"
           << "  mf_u64 base = ((mf_u64)blockIdx.x * MF_BLOCK + threadIdx.x) * " << V << ";\n";
         for (int k : out.used_inputs)
@@ -2397,6 +2426,26 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
         s << "  if (aborted && threadIdx.x == 0) {\n    atomicOr(status, 1u);\n"
           << "    for (unsigned k = it; k < issued; k++) mf_mbar_wait_bounded(&mf_bar[k % MF_STAGES], (k / MF_STAGES) & 1u);\n"
           << "  }\n";
+      } else if (first) {
+        s << "  for (; base < stride; base += step) {\n    const mf_u64 ahead = base + step;\n";
+        for (int k : raw_cols)
+          s << "    const " << RT << " s" << k << " = c" << k << ";\n    c" << k << " = ahead < stride ? "
+            << raw_at(k, "ahead") << " : " << RT << "();\n";
+        for (size_t m = 0; m < fold.cols.size(); m++) {
+          s << "    " << VT << " l" << m << ";\n    {\n";
+          for (int v = 0; v < V; v++) {
+            const std::string y = "y" + std::to_string(v), w = "w" + std::to_string(v);
+            emit_fold(s, "      ", y, fold.cols[m],
+                      [&](int k) { return "s" + std::to_string(k) + (V == 1 ? "" : v == 0 ? ".x" : ".y"); });
+            s << "      const mf_dw " << w << " = mf_dw_split(" << y << ");\n";
+          }
+          s << "      l" << m << " = "
+            << (V == 1 ? "make_float2(w0.h, w0.l)" : "make_float4(w0.h, w0.l, w1.h, w1.l)") << ";\n    }\n"
+            << "    *reinterpret_cast<" << VT << "*>(prepared + (mf_u64)" << m << " * stride + base) = l" << m << ";\n";
+        }
+        s << "    if (base < n) {\n";
+        emit_events(s, "      ", "base", nullptr);
+        s << "    }\n  }\n";
       } else if (prefetch) {
         if (out.stages > 1) s << "#pragma unroll " << out.stages << "\n";
         s << "  for (; base < n; base += step) {\n    const mf_u64 ahead = base + step;\n";
@@ -2496,8 +2545,8 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
     if (threadIdx.x == 0) *reinterpret_cast<volatile unsigned*>(status + 1) = seq;
   }
 )CUDA";
+    const std::string lone_tail = s.str().substr(size_t(body_mark) + lone_work.str().size());
     if (!out.pipelined) {
-      const std::string tail = s.str().substr(size_t(body_mark) + lone_work.str().size());
       auto resident = [&](std::string work) {
         replace_all(work, "blockIdx.x", "mf_vb");
         replace_all(work, "gridDim.x", "mf_grid");
@@ -2509,10 +2558,32 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
       };
       out.resident_prefix = s.str().substr(0, size_t(entry_mark));
       out.resident_data_type = DT;
-      out.resident_body = resident(lone_work.str() + tail);
-      out.resident_plain = resident(part_work.str() + tail);
+      out.resident_body = resident(lone_work.str() + lone_tail);
+      out.resident_plain = resident(part_work.str() + lone_tail);
     }
     s << "}\n";
+    // ---- the first evaluation of a dataset ----
+    // Preparing the columns in a pass of its own writes them only for the
+    // event loop to read them again. This entry is the event loop over the
+    // columns as they are: each thread prepares the events it evaluates (the
+    // padding up to `stride` as well) and stores them for the evaluations to
+    // come. The same events, operations and grid as the entry above, so the
+    // same sums bit for bit. Bound by the columns' bytes and by latency at 16
+    // warps per SM: for 1M K*mumu P-wave events (88 MB read, 72 MB written)
+    // the pass and the gradient took 20.2 + 18.4 us (ncu), this entry 32.4
+    // with the next columns' loads in flight and 36 without; a new dataset
+    // with its precompute and first gradient 111.5 -> 98.9 us. For
+    // gradient-sized kernels; Hessians are issue-bound and seldom first.
+    out.first = prep && pair && ar == Ar::DW && !st32 && !out.pipelined && NC > 0 && M <= 16;
+    if (out.first) {
+      std::ostringstream first_work;
+      block_work(first_work, false, true);
+      s << "extern \"C\" __global__ void MF_BOUNDS " << out.entry
+        << "_first(const double* __restrict__ raw, mf_u64 stride, mf_u64 n, mf_args P, float2* __restrict__ partials,"
+        << " unsigned* __restrict__ counter, double* __restrict__ out, unsigned* __restrict__ status, unsigned seq, "
+        << DT << "* __restrict__ prepared) {\n"
+        << first_work.str() << lone_tail << "}\n";
+    }
     // ---- batched evaluations: per-block partials only, then one combine ----
     // Evaluation e of a batch writes its partial rows to its own slot of the
     // batch's partial buffer without counting or combining, so consecutive
@@ -2693,18 +2764,9 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
         return "(double)__ldg(data + (mf_u64)" + std::to_string(col) + " * stride + i)";
       };
       for (size_t m = 0; m < fold.cols.size(); m++) {
-        const auto& terms = fold.cols[m];
-        s << "    {\n      double y = 0.0;\n      if (v) {\n        y = " << src(terms[0].first) << ";\n";
-        for (size_t t = 1; t < terms.size(); t++) {
-          const double c = terms[t].second;
-          if (c == 1.0)
-            s << "        y = __dadd_rn(y, " << src(terms[t].first) << ");\n";
-          else if (c == -1.0)
-            s << "        y = __dsub_rn(y, " << src(terms[t].first) << ");\n";
-          else
-            s << "        y = __fma_rn(" << fmt_const(c, false) << ", " << src(terms[t].first) << ", y);\n";
-        }
-        s << "      }\n";
+        s << "    {\n      double y = 0.0;\n      if (v) {\n";
+        emit_fold(s, "        ", "f", fold.cols[m], src);
+        s << "        y = f;\n      }\n";
         if (pair)
           s << "      const mf_dw w = mf_dw_split(y);\n      outp[(mf_u64)" << m << " * stride + i] = make_float2(w.h, w.l);\n";
         else

@@ -92,6 +92,7 @@ struct LoweredKernel {
   std::vector<int> used_inputs;  // input columns read by the kernel
   int vec = 1;                   // events per thread per iteration
   int block = 256;
+  bool first = false;      // REDUCE: has an entry that prepares a dataset as it evaluates it
   unsigned gen_chunk = 1;  // GENERATE: largest number of proposals a thread tests in a row
   int acc_reg = 0;               // REDUCE: outputs whose per-thread partials are registers (the rest: shared memory)
   // REDUCE kernels stream tiles of `tile` events through `stages` shared-memory

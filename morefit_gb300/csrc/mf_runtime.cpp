@@ -316,6 +316,7 @@ struct mf_kernel {
   std::shared_ptr<LoadedModule> module;
   cudaKernel_t fn = nullptr;
   cudaKernel_t fn_seg = nullptr;
+  cudaKernel_t fn_first = nullptr;  // REDUCE kernels that can prepare a dataset as they evaluate it
   cudaKernel_t fn_prep = nullptr;  // REDUCE kernels reading prepared columns
   cudaKernel_t fn_part = nullptr;     // REDUCE: per-block partials only (batched evaluations)
   cudaKernel_t fn_combine = nullptr;  // REDUCE: one block per batched evaluation
@@ -335,7 +336,7 @@ struct mf_kernel {
 namespace mfi {
 int launch_reduce(mf_kernel* k, const void* data, uint64_t stride, uint64_t n, const double* params,
                   double* partials, unsigned* counter, double* out, cudaStream_t stream, int grid_cap,
-                  bool dependent = false, unsigned seq = 0);
+                  bool dependent = false, unsigned seq = 0, const void* raw = nullptr);
 }
 
 // ---------------------------------------------------------------- helpers --
@@ -502,13 +503,27 @@ uint64_t prep_key(const mf_kernel* k) {
   return h;
 }
 
+void mark_prepared(mf_derived* d, const mf_buffer* in, uint64_t stride) {
+  d->gen = in->gen;
+  d->n = stride;
+  d->stride = stride;
+}
+
+// Whether an evaluation's grid, sized for its n events, is large enough for
+// all `stride` rows of the columns.
+bool whole_columns(uint64_t stride, uint64_t n) { return stride - n <= n / 8 + 4096; }
+
 // The device columns kernel `k` reads for input buffer `in`: the buffer
 // itself, or its prepared copy, (re)made on the context's stream when the
 // buffer was written since (or the column stride changed). The copy covers
 // all `stride` rows of the columns, so evaluations of any event count or
 // segment of the buffer share it (event loops never accumulate rows at or
 // beyond their n).
-int prepare_input(const mf_kernel* k, const mf_buffer* in, uint64_t stride, const void** data) {
+// `stale` (may be null): a caller that goes on to one evaluation of the whole
+// buffer by the _first entry gets, if the copy has to be made, its slot there
+// instead (with the memory for it), and marks it made once that is launched.
+int prepare_input(const mf_kernel* k, const mf_buffer* in, uint64_t stride, const void** data,
+                  mf_derived** stale = nullptr) {
   if (!k->lowered.prep) {
     *data = in->ptr;
     return MF_OK;
@@ -544,6 +559,11 @@ int prepare_input(const mf_kernel* k, const mf_buffer* in, uint64_t stride, cons
     d->bytes = need;
     c->allocated += need;
   }
+  *data = d->ptr;
+  if (stale && k->fn_first) {
+    *stale = d;
+    return MF_OK;
+  }
   const uint64_t blocks = (stride + 255) / 256;
   const int grid = int(std::max<uint64_t>(1, std::min<uint64_t>(blocks, uint64_t(c->num_sms) * 16)));
   const void* src = in->ptr;
@@ -552,10 +572,7 @@ int prepare_input(const mf_kernel* k, const mf_buffer* in, uint64_t stride, cons
   void* args[] = {const_cast<void**>(&src), &stride, &rows, &dst};
   res_yield(c);
   MF_CUDA_TRY(cudaLaunchKernel(reinterpret_cast<const void*>(k->fn_prep), dim3(grid), dim3(256), args, 0, c->stream));
-  d->gen = in->gen;
-  d->n = stride;
-  d->stride = stride;
-  *data = d->ptr;
+  mark_prepared(d, in, stride);
   return MF_OK;
 }
 
@@ -940,6 +957,8 @@ int mf_kernel_build(mf_context* c, const mf_kernel_desc* d, mf_kernel** out) {
     MF_CUDA_TRY(cudaLibraryGetKernel(&k->fn_seg, k->module->lib, (k->lowered.entry + "_segments").c_str()));
   if (d->kind == MF_KERNEL_REDUCE) {
     MF_CUDA_TRY(cudaLibraryGetKernel(&k->fn_part, k->module->lib, (k->lowered.entry + "_part").c_str()));
+    if (k->lowered.first)
+      MF_CUDA_TRY(cudaLibraryGetKernel(&k->fn_first, k->module->lib, (k->lowered.entry + "_first").c_str()));
     if (k->lowered.batch_max)
       MF_CUDA_TRY(cudaLibraryGetKernel(&k->fn_batch, k->module->lib, (k->lowered.entry + "_batch").c_str()));
     MF_CUDA_TRY(cudaLibraryGetKernel(&k->fn_combine, k->module->lib, (k->lowered.entry + "_combine").c_str()));
@@ -1433,7 +1452,7 @@ int grid_for(const mf_kernel* k, uint64_t n) {
 // waits for it before it touches the shared scratch.
 int launch_reduce(mf_kernel* k, const void* data, uint64_t stride, uint64_t n, const double* params,
                   double* partials, unsigned* counter, double* out, cudaStream_t stream, int grid_cap,
-                  bool dependent, unsigned seq) {
+                  bool dependent, unsigned seq, const void* raw) {
   int grid = grid_for(k, n);
   if (grid_cap > 0) grid = std::min(grid, grid_cap);
   // argument struct: parameter-only values evaluated here, pre-rounded for the kernel's arithmetic
@@ -1445,7 +1464,9 @@ int launch_reduce(mf_kernel* k, const void* data, uint64_t stride, uint64_t n, c
     return fail(MF_ERR_INVALID, std::string("parameter evaluation: ") + e.what());
   }
   unsigned* status = k->ctx->status;
-  void* args[] = {const_cast<void**>(&data), &stride, &n, pv.data(), &partials, &counter, &out, &status, &seq};
+  // raw (the _first entry): the unprepared columns; `data` is then written
+  void* args[] = {const_cast<void**>(raw ? &raw : &data), &stride, &n, pv.data(), &partials, &counter, &out, &status,
+                  &seq, const_cast<void**>(&data)};
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(k->lowered.block);
@@ -1457,7 +1478,7 @@ int launch_reduce(mf_kernel* k, const void* data, uint64_t stride, uint64_t n, c
   cfg.attrs = attr;
   cfg.numAttrs = dependent ? 1 : 0;
   res_yield(k->ctx);
-  MF_CUDA_TRY(cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(k->fn), args));
+  MF_CUDA_TRY(cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(raw ? k->fn_first : k->fn), args));
   return MF_OK;
 }
 
@@ -1677,12 +1698,14 @@ static int reduce_direct(mf_kernel* k, const mf_buffer* in, uint64_t stride, uin
   if (rc) return rc;
   *c->status_host = 0u;
   const void* data = nullptr;
-  rc = prepare_input(k, in, stride, &data);
+  mf_derived* stale = nullptr;
+  rc = prepare_input(k, in, stride, &data, whole_columns(stride, n) ? &stale : nullptr);
   if (rc) return rc;
   if (++c->sync_seq == 0u) c->sync_seq = 1u;  // 0 means "asynchronous" to the kernel
   rc = mfi::launch_reduce(k, data, stride, n, params, c->partials, c->counter, c->out_dev, c->stream, 0, false,
-                          c->sync_seq);
+                          c->sync_seq, stale ? in->ptr : nullptr);
   if (rc) return rc;
+  if (stale) mark_prepared(stale, in, stride);
   rc = wait_sync_word(c, c->sync_seq);
   if (rc) return rc;
   std::memcpy(sums, c->out_host, k->n_outputs * sizeof(double));
@@ -2275,9 +2298,13 @@ int mf_kernel_reduce_async(mf_kernel* k, const mf_buffer* in, uint64_t stride, u
   if (rc) return rc;
   double* dst = static_cast<double*>(out->ptr) + out_index * k->n_outputs;
   const void* data = nullptr;
-  rc = prepare_input(k, in, stride, &data);
+  mf_derived* stale = nullptr;
+  rc = prepare_input(k, in, stride, &data, whole_columns(stride, n) ? &stale : nullptr);
   if (rc) return rc;
-  return mfi::launch_reduce(k, data, stride, n, params, c->partials, c->counter, dst, c->stream, 0);
+  rc = mfi::launch_reduce(k, data, stride, n, params, c->partials, c->counter, dst, c->stream, 0, false, 0,
+                          stale ? in->ptr : nullptr);
+  if (rc == MF_OK && stale) mark_prepared(stale, in, stride);
+  return rc;
 }
 
 int mf_kernel_reduce_many(mf_kernel* k, uint32_t count, const mf_buffer* const* inputs, const uint64_t* strides,
