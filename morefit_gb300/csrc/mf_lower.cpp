@@ -949,11 +949,15 @@ __device__ __forceinline__ mf_dw mf_dw_shfl_xor(mf_dw a, int o) {
 // mf_sum_rows: the sums of `nb` partial rows, `step` rows apart, into sums[]
 // (shared, complete for every thread on return). Thread (g, o) takes rows g,
 // g + MF_GRP, ... of output o, so that a warp's loads are contiguous and a
-// round of loads covers MF_Q rows per thread, added as a tree; then MF_GRP
-// partials per output are added in order (few) or by a warp. Measured as part of a lone launch,
-// one thread per row and a shuffle tree per output took 18 us of the P-wave
-// Hessian's 54 (36 outputs, 152 rows, ncu) and 100 of the S+P wave's 163
-// (105 outputs, 608 rows).
+// round of loads covers MF_Q rows per thread, added as a tree; then the MF_GRP
+// (at most 32) partials per output are added as a tree, by one thread (few) or
+// a warp. Measured as part of a lone launch, one thread per row and a shuffle
+// tree per output took 18 us of the P-wave Hessian's 54 (36 outputs, 152 rows,
+// ncu) and 100 of the S+P wave's 163 (105 outputs, 608 rows). A lone small
+// evaluation waits for every add in turn (about 60 cycles): trees instead of
+// chains here and across a block's warps, and no tree of empty rows for grids
+// of up to MF_GRP blocks, 14.6 -> 14.3 us (P-wave NLL in FP32, 30011 events)
+// and 15.7 -> 15.3 (mass gradient, 1000).
 const char* kCombine = R"CUDA(
 template <int N> __device__ __forceinline__ void mf_warp_sums(mf_dw (&v)[N], int lane) {
   int o = 16;
@@ -969,6 +973,26 @@ template <int N> __device__ __forceinline__ void mf_warp_sums(mf_dw (&v)[N], int
 #pragma unroll
   for (; o > 0; o >>= 1) v[0] = mf_dw_add(v[0], mf_dw_shfl_xor(v[0], o));
 }
+// t[0] = the sum of t[0..N)
+template <int N> __device__ __forceinline__ void mf_tree_sum(mf_dw (&t)[N]) {
+#pragma unroll
+  for (int s = 1; s < N; s *= 2)
+#pragma unroll
+    for (int q = 0; q + s < N; q += 2 * s) t[q] = mf_dw_add(t[q], t[q + s]);
+}
+// the sum of one output over the block's warps (rows of MF_NOUT), in eights
+__device__ __forceinline__ mf_dw mf_sum_warps(const float2* p) {
+  mf_dw a;
+  for (int w0 = 0; w0 < MF_BLOCK / 32; w0 += 8) {
+    mf_dw t[MF_BLOCK / 32 < 8 ? MF_BLOCK / 32 : 8];
+#pragma unroll
+    for (int w = 0; w < (MF_BLOCK / 32 < 8 ? MF_BLOCK / 32 : 8); w++)
+      t[w] = w0 + w < MF_BLOCK / 32 ? mf_dw_pair(p[(w0 + w) * MF_NOUT]) : mf_dw_make(0.0f, 0.0f);
+    mf_tree_sum(t);
+    a = w0 == 0 ? t[0] : mf_dw_add(a, t[0]);
+  }
+  return a;
+}
 __device__ __forceinline__ void mf_sum_rows(const float2* rows, unsigned nb, unsigned step, float2* part, float2* sums) {
   const mf_u64 stride = (mf_u64)step * MF_NOUT;
 #if MF_GRP > 1
@@ -978,22 +1002,23 @@ __device__ __forceinline__ void mf_sum_rows(const float2* rows, unsigned nb, uns
   const int g = 0;
   for (int o = threadIdx.x; o < MF_NOUT; o += MF_BLOCK) {
 #endif
-    mf_dw a = mf_dw_make(0.0f, 0.0f);
-    for (unsigned r0 = g; r0 < nb; r0 += MF_GRP * MF_Q) {
-      float2 v[MF_Q];
+    mf_dw a;
+    if (nb <= MF_GRP) {  // a row each at most
+      a = g < nb ? mf_dw_pair(__ldcg(rows + g * stride + o)) : mf_dw_make(0.0f, 0.0f);
+    } else {
+      for (unsigned r0 = g; r0 == g || r0 < nb; r0 += MF_GRP * MF_Q) {
+        float2 v[MF_Q];
 #pragma unroll
-      for (int q = 0; q < MF_Q; q++) {
-        const unsigned r = r0 + q * MF_GRP;
-        v[q] = r < nb ? __ldcg(rows + r * stride + o) : make_float2(0.0f, 0.0f);
+        for (int q = 0; q < MF_Q; q++) {
+          const unsigned r = r0 + q * MF_GRP;
+          v[q] = r < nb ? __ldcg(rows + r * stride + o) : make_float2(0.0f, 0.0f);
+        }
+        mf_dw t[MF_Q];
+#pragma unroll
+        for (int q = 0; q < MF_Q; q++) t[q] = mf_dw_pair(v[q]);
+        mf_tree_sum<MF_Q>(t);
+        a = r0 == g ? t[0] : mf_dw_add(a, t[0]);
       }
-      mf_dw t[MF_Q];
-#pragma unroll
-      for (int q = 0; q < MF_Q; q++) t[q] = mf_dw_pair(v[q]);
-#pragma unroll
-      for (int h = MF_Q / 2; h > 0; h >>= 1)
-#pragma unroll
-        for (int q = 0; q < h; q++) t[q] = mf_dw_add(t[q], t[q + h]);
-      a = mf_dw_add(a, t[0]);
     }
 #if MF_GRP > 1
     part[g * MF_NOUT + o] = make_float2(a.h, a.l);
@@ -1001,19 +1026,19 @@ __device__ __forceinline__ void mf_sum_rows(const float2* rows, unsigned nb, uns
   __syncthreads();
 #if MF_GRP <= 8
   if (threadIdx.x < MF_NOUT) {
-    mf_dw a = mf_dw_pair(part[threadIdx.x]);
+    mf_dw t[MF_GRP];
 #pragma unroll
-    for (int q = 1; q < MF_GRP; q++) a = mf_dw_add(a, mf_dw_pair(part[q * MF_NOUT + threadIdx.x]));
-    sums[threadIdx.x] = make_float2(a.h, a.l);
+    for (int q = 0; q < MF_GRP; q++) t[q] = mf_dw_pair(part[q * MF_NOUT + threadIdx.x]);
+    mf_tree_sum<MF_GRP>(t);
+    sums[threadIdx.x] = make_float2(t[0].h, t[0].l);
   }
 #else
   for (int j = threadIdx.x >> 5; j < MF_NOUT; j += MF_BLOCK / 32) {
-    mf_dw a = mf_dw_make(0.0f, 0.0f);
+    const int q = threadIdx.x & 31;
+    mf_dw a = q < MF_GRP ? mf_dw_pair(part[q * MF_NOUT + j]) : mf_dw_make(0.0f, 0.0f);
 #pragma unroll
-    for (int q = threadIdx.x & 31; q < MF_GRP; q += 32) a = mf_dw_add(a, mf_dw_pair(part[q * MF_NOUT + j]));
-#pragma unroll
-    for (int w = 16; w > 0; w >>= 1) a = mf_dw_add(a, mf_dw_shfl_xor(a, w));
-    if ((threadIdx.x & 31) == 0) sums[j] = make_float2(a.h, a.l);
+    for (int w = MF_GRP > 16 ? 16 : 8; w > 0; w >>= 1) a = mf_dw_add(a, mf_dw_shfl_xor(a, w));
+    if (q == 0) sums[j] = make_float2(a.h, a.l);
   }
 #endif
 #else
@@ -1383,10 +1408,10 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
   s << "#define MF_NREG " << NREG << "\n";
   // launch bounds of the event-loop entries
   s << "#define MF_BOUNDS __launch_bounds__(MF_BLOCK)\n";
-  // combine of block partial rows: MF_GRP threads share an output's rows, each
+  // combine of block partial rows: MF_GRP threads (a warp's lanes at most) share an output's rows, each
   // with MF_Q loads in flight; kernels of many outputs, whose grids of small
   // blocks leave hundreds of rows, combine them in groups of MF_ROWS blocks first
-  const int grp = std::max(1, out.block / M);
+  const int grp = std::max(1, std::min(32, out.block / M));
   int q = 2;  // a power of two: the rows of a round are added as a tree
   while (q < 16 && q * grp < 608) q *= 2;
   s << "#define MF_GRP " << grp << "\n#define MF_Q " << q << "\n";
@@ -2269,8 +2294,7 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
       warp_reduce(o);
       o << "  __syncthreads();\n"
         << "  for (int j = threadIdx.x; j < MF_NOUT; j += MF_BLOCK) {\n"
-        << "    mf_dw a = mf_dw_pair(mf_part[j]);\n"
-        << "#pragma unroll\n    for (int w = 1; w < MF_BLOCK / 32; w++) a = mf_dw_add(a, mf_dw_pair(mf_part[w * MF_NOUT + j]));\n"
+        << "    const mf_dw a = mf_sum_warps(mf_part + j);\n"
         << "    mf_blk[j] = make_float2(a.h, a.l);\n  }\n  __syncthreads();\n";
     };
     bool f32_logprod = false;
@@ -2647,9 +2671,7 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
   for (unsigned q = threadIdx.x; q < (last - first) * MF_NOUT; q += MF_BLOCK) {
     const unsigned e = q / MF_NOUT, j = q - e * MF_NOUT;
     if (blockIdx.x >= B.job[first + e].grid) continue;
-    mf_dw a = mf_dw_pair(mf_warps[e][j]);
-#pragma unroll
-    for (int w = 1; w < MF_BLOCK / 32; w++) a = mf_dw_add(a, mf_dw_pair(mf_warps[e][w * MF_NOUT + j]));
+    const mf_dw a = mf_sum_warps(mf_warps[e] + j);
     partials_all[(first + e) * pstride + (mf_u64)blockIdx.x * MF_NOUT + j] = make_float2(a.h, a.l);
   }
 }
