@@ -2615,7 +2615,16 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
     // its own work); <entry>_combine then reduces every evaluation's rows
     // (one block each, the same fixed order: the sums equal the
     // single-evaluation entry's).
-    s << "extern \"C\" __global__ void MF_BOUNDS " << out.entry << "_part(const " << DT
+    //
+    // Consecutive grids of two blocks per SM overlap in the slot of a third
+    // where the registers leave one: asked for (80 registers) where one
+    // vector of the columns and the partials take at most 56, which costs the
+    // P-wave gradient 12 bytes of spill. Datasets in turn from HBM, 1M events:
+    // 13.2 us an evaluation at the 86 registers it takes of itself, 11.0 at
+    // 80. The S+P wave (24 columns) would spill its events.
+    const bool three = ar == Ar::DW && out.block == 256 && NC > 1 && 2 * (NC * V + M) <= 56;
+    s << "extern \"C\" __global__ void " << (three ? "__launch_bounds__(MF_BLOCK, 3) " : "MF_BOUNDS ") << out.entry
+      << "_part(const " << DT
       << "* __restrict__ data, mf_u64 stride, mf_u64 n, mf_args P, float2* __restrict__ partials,"
       << " unsigned* __restrict__ status) {\n"
       << part_work.str()
