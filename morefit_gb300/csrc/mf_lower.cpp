@@ -2737,12 +2737,14 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
       load_table(o);
       prologue(o, "P.");
       acc_decl(o);
-      o << "  for (unsigned i = threadIdx.x; i < cnt; i += MF_BLOCK) {\n";
+      // from the last turn to cnt itself: i + MF_BLOCK would wrap for counts
+      // near 2^32, and the loop not end
+      o << "  for (unsigned i = threadIdx.x; i < cnt; i = cnt - i > MF_BLOCK ? i + MF_BLOCK : cnt) {\n";
       if (seg_prefetch) {
         for (int k : out.used_inputs) o << "    const " << DT << " l" << k << " = c" << k << ";\n";
-        o << "    const unsigned ahead = i + MF_BLOCK;\n";
+        o << "    const bool more = cnt - i > MF_BLOCK;\n";
         for (int k : out.used_inputs)
-          o << "    c" << k << " = ahead < cnt ? " << load_event(k, "ahead") << " : " << DT << "();\n";
+          o << "    c" << k << " = more ? " << load_event(k, "(i + MF_BLOCK)") << " : " << DT << "();\n";
       }
       for (int k : out.used_inputs)
         o << "    const " << XT << " x" << k << " = "
