@@ -2938,6 +2938,13 @@ __device__ __forceinline__ mf_rng mf_rng_spread(mf_rng st, unsigned steps, unsig
     // them, when the stream is complete (full warps instead of the few lanes
     // that accept).
     const bool filter = !ar32;
+    // A bound as an FP32 literal, 0 or at least 2^-126: a smaller one is out of
+    // range for the compiler, and results that underflow are off by up to 2^-150.
+    auto bound_f = [](double e) {
+      char b[48];
+      std::snprintf(b, sizeof b, "%.9ef", e > 0.0 ? e + 0x1p-126 : 0.0);
+      return std::string(b);
+    };
     std::string filter_call;
     std::vector<int> filter_uniform;
     if (filter) {
@@ -2959,11 +2966,10 @@ __device__ __forceinline__ mf_rng mf_rng_spread(mf_rng st, unsigned steps, unsig
         const Node& n = ns[id];
         if (n.op == Op::Const) {
           const float v = float(n.value);
+          if (!std::isfinite(v)) return "mf_ef_make(0.0f, MF_EF_INF)";  // decided in FP64
           // the rounding of the constant, bounded (0 when it is exact)
-          const double e = std::isfinite(v) ? std::fabs(n.value - double(v)) * 1.0000005 : 0.0;
-          char b[96];
-          std::snprintf(b, sizeof b, "mf_ef_make(%s, %.9ef)", fmt_const(n.value, true).c_str(), e);
-          return b;
+          const double e = std::fabs(n.value - double(v)) * 1.0000005;
+          return "mf_ef_make(" + fmt_const(n.value, true) + ", " + bound_f(e) + ")";
         }
         if (n.op == Op::Input) return "x" + std::to_string(n.index);
         return (n.uniform ? "uf" : "f") + std::to_string(id);
@@ -3040,10 +3046,13 @@ __device__ __forceinline__ mf_rng mf_rng_spread(mf_rng st, unsigned steps, unsig
       if (filter) {
         for (int d = 0; d < D; d++) {
           const double lo = printed15(gen->lo[d]), del = printed15(gen->hi[d] - gen->lo[d]);
-          char eb[48];
-          std::snprintf(eb, sizeof eb, "%.9ef", (std::fabs(lo) + std::fabs(del)) * 0x1p-22);
-          s << "        const mf_ef xe" << d << " = mf_ef_make(__fmaf_rn(" << fmt_const(del, true) << ", (float)d" << d
-            << " * 2.3283064365386963e-10f, " << fmt_const(lo, true) << "), " << eb << ");\n";
+          // an end or a width that FP32 cannot hold: decided in FP64
+          const bool fits = std::isfinite(float(lo)) && std::isfinite(float(del)) && std::isfinite(float(lo + del));
+          s << "        const mf_ef xe" << d << " = mf_ef_make("
+            << (fits ? "__fmaf_rn(" + fmt_const(del, true) + ", (float)d" + std::to_string(d) +
+                           " * 2.3283064365386963e-10f, " + fmt_const(lo, true) + ")"
+                     : std::string("0.0f"))
+            << ", " << (fits ? bound_f((std::fabs(lo) + std::fabs(del)) * 0x1p-22) : "MF_EF_INF") << ");\n";
         }
         s << "        bool amb = false;\n        const mf_ef p = " << filter_call << ";\n"
           << "        const mf_ef ug = mf_ef_mul(maxprob_f, mf_ef_make((float)d" << D
