@@ -24,7 +24,6 @@ the covariance to -2 H^-1 F H^-1 (fitter.hh:894-943). ``fisher()`` and
 from __future__ import annotations
 
 import ast
-import functools
 import json
 import re
 from pathlib import Path
@@ -54,12 +53,18 @@ def weighted_covariance(hessian: np.ndarray, fisher: np.ndarray) -> np.ndarray:
     return -2.0 * hinv @ np.asarray(fisher, dtype=np.float64) @ hinv
 
 
-@functools.lru_cache(maxsize=1024)
+# Longer texts are compared as they are: reading the S+P wave's 148 buffers (220
+# kB) into trees took 0.2 s of a process's first combined kernel, and this limit
+# shares the same 14 of its buffers (and all of the other models') in 0.7 ms.
+DEFINITION_MAX = 200
+
+
 def _definition(text: str):
     """What a parameter buffer's expression computes, as a comparable value in
     which the operand order of a sum or product does not matter (exactly the
-    same double either way); the text itself where it holds a conditional."""
-    if "?" in text:
+    same double either way); the text itself where it holds a conditional or
+    more than DEFINITION_MAX characters."""
+    if len(text) > DEFINITION_MAX or "?" in text:
         return text
 
     def key(n):
@@ -74,8 +79,18 @@ def _definition(text: str):
         return n.value if isinstance(n, ast.Constant) else n.id
     try:
         return key(ast.parse(text, mode="eval").body)
-    except (SyntaxError, AttributeError):
+    except (SyntaxError, AttributeError, RecursionError):  # the last from a caller deep in its stack
         return text
+
+
+def _combined_buffers(gbuf, hbuf, share: bool):
+    """Names of the Hessian's parameter buffers beside the gradient's in one
+    kernel, and those that have to be added: each gets a name of its own, or
+    (share) the gradient's where that holds the same definition."""
+    known = {_definition(e): n for n, e in gbuf} if share else {}
+    own = {n: n.replace("morefit_", "mfh_") for n, _ in hbuf}
+    names = {n: known.get(_definition(e), own[n]) if share else own[n] for n, e in hbuf}
+    return names, [n for n, _ in hbuf if names[n] == own[n]]
 
 
 class Likelihood:
@@ -344,12 +359,11 @@ class Likelihood:
         # then share the subexpressions built on them (the Crystal Ball's
         # powers and exponentials, the P-wave density's dot product). Not in
         # FP32 arithmetic, whose last bit follows the text's own operations.
-        known = {_definition(e): n for n, e in gbuf} if self.kernelT == np.float64 else {}
-        names = {n: known.get(_definition(e), n.replace("morefit_", "mfh_")) for n, e in hbuf}
+        names, added = _combined_buffers(gbuf, hbuf, self.kernelT == np.float64)
 
         def ren(e):
             return re.sub(r"\bmorefit_parambuffer_\d+\b", lambda m: names.get(m.group(0), m.group(0)), e)
-        hb = [(names[n], ren(e)) for n, e in hbuf if names[n].startswith("mfh_")]
+        hb = [(names[n], ren(e)) for n, e in hbuf if n in added]
         params = list(g["params"]) + [n for n, _ in hb]
         exprs = list(g["exprs"]) + [ren(e) for e in h["exprs"]]
         defs = dict(gbuf)
