@@ -2433,6 +2433,9 @@ int mf_kernel_reduce_segments(mf_kernel* k, const mf_buffer* in, uint64_t stride
                                c->stream));
   MF_CUDA_TRY(cudaStreamSynchronize(c->stream));
   std::memcpy(sums, c->out_host, size_t(nseg) * k->n_outputs * sizeof(double));
+  // the sums of no events are zero; 0 times a factor that is not finite is not
+  for (uint32_t s = 0; s < nseg; s++)
+    if (seg_count[s] == 0) std::fill_n(sums + size_t(s) * k->n_outputs, k->n_outputs, 0.0);
   if (!k->desc) return MF_OK;
   // Segments whose double-float sums are non-finite: again in native FP64.
   std::vector<uint32_t> bad;
