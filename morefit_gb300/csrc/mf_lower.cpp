@@ -1684,7 +1684,7 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
             u = n.a;
             sg = 1;
           }
-          if (x >= 0 && !skip[x]) {
+          if (x >= 0 && !skip[x] && !chains.count(x)) {
             addu[j] = u;
             addsign[j] = sg;
             skip[r] = 1;
@@ -1701,76 +1701,6 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
           lognode[j] = lg;
           skip[r] = 1;
           skip[lg] = 1;
-        }
-      }
-    }
-    // Double-float REDUCE bodies: sums of three and more terms, or of products
-    // used nowhere else, as one lazily renormalized sum (a product costs 12
-    // operations there instead of 7 and an 11-operation addition), and outputs
-    // that are such sums straight into their accumulators. Batched, 1M events:
-    // mass Hessian 46.9 -> 40.1 us; Crystal Ball F + gradient + Hessian, 250k:
-    // 45.6 -> 40.4; the errors against 64 bits stay the same. (Products left
-    // unnormalized for such sums would save 5% more, but the mass Hessian's
-    // error grew from 3.1e-12 to 4.5e-12.)
-    struct Term {
-      int a, b;  // a product, or (b < 0) a value
-      bool minus;
-    };
-    std::map<int, std::vector<Term>> sums;          // node -> its terms
-    std::vector<std::vector<Term>> outsum(roots.size());  // output -> the terms it accumulates
-    if (ar == Ar::DW && kind == Kind::Reduce) {
-      auto body_node = [&](int k) { return k >= 0 && live[k] && !ns[k].uniform && ns[k].op != Op::Input; };
-      auto open = [&](int k) {  // an addition whose statement may be taken apart
-        return body_node(k) && (ns[k].op == Op::Add || ns[k].op == Op::Sub) && !skip[k] && !chains.count(k);
-      };
-      std::function<void(int, bool, bool, std::vector<Term>&, std::vector<int>&)> take =
-          [&](int k, bool minus, bool top, std::vector<Term>& t, std::vector<int>& gone) {
-            const bool once = top || uses[k] == 1;
-            if (once && open(k)) {
-              if (!top) gone.push_back(k);
-              take(ns[k].a, minus, false, t, gone);
-              take(ns[k].b, minus != (ns[k].op == Op::Sub), false, t, gone);
-            } else if (once && body_node(k) && ns[k].op == Op::Neg && !skip[k]) {
-              gone.push_back(k);
-              take(ns[k].a, !minus, false, t, gone);
-            } else if (once && body_node(k) && ns[k].op == Op::Mul && !skip[k]) {
-              gone.push_back(k);
-              t.push_back({ns[k].a, ns[k].b, minus});
-            } else {
-              t.push_back({k, -1, minus});
-            }
-          };
-      std::map<int, int> output_of;  // node only output j uses, which j accumulates as it is
-      for (size_t j = 0; j < roots.size(); j++) {
-        const int r = accnode[j];
-        if (fused[j].first < 0 && logprod[j] < 0 && body_node(r) && uses[r] == 1) output_of[r] = int(j);
-      }
-      for (size_t q = ns.size(); q-- > 0;) {
-        const int i = int(q);
-        auto out_it = output_of.find(i);
-        if (out_it != output_of.end() && chains.count(i)) {
-          for (auto& [a, b] : chains.at(i)) outsum[out_it->second].push_back({a, b, false});
-          chains.erase(i);
-          skip[i] = 1;
-          continue;
-        }
-        if (!open(i)) continue;
-        std::vector<Term> t;
-        std::vector<int> gone;
-        take(i, false, true, t, gone);
-        int plain = -11, lazily = 6;  // operations as statements, and as one sum
-        for (size_t m = 0; m < t.size(); m++) {
-          plain += 11 + (t[m].b >= 0 ? 7 : 0);
-          lazily += t[m].b >= 0 ? (m ? 12 : 4) : (m ? 8 : 0);
-        }
-        const bool output = out_it != output_of.end();
-        if (!output && lazily >= plain) continue;
-        for (int g : gone) skip[g] = 1;
-        if (output) {
-          outsum[out_it->second] = t;
-          skip[i] = 1;
-        } else {
-          sums[i] = t;
         }
       }
     }
@@ -1856,19 +1786,6 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
         for (auto& [ta, tb] : ch->second)
           c += (&ta == &ch->second.front().first ? " mf_dw t_ = mf_dw_prod(" : " mf_dw_acc_mul(t_, ") + eref(ta) + ", " +
                eref(tb) + ");";
-        return c + " e" + std::to_string(id) + " = mf_dw_renorm(t_); }";
-      }
-      auto sm = sums.find(id);
-      if (sm != sums.end()) {
-        std::string c = "mf_dw e" + std::to_string(id) + "; { mf_dw t_ = ";
-        for (size_t m = 0; m < sm->second.size(); m++) {
-          const Term& t = sm->second[m];
-          const std::string x = t.minus ? "mf_dw_neg(" + eref(t.a) + ")" : eref(t.a);
-          if (m == 0)
-            c += t.b >= 0 ? "mf_dw_prod(" + x + ", " + eref(t.b) + ");" : x + ";";
-          else
-            c += t.b >= 0 ? " mf_dw_acc_mul(t_, " + x + ", " + eref(t.b) + ");" : " mf_dw_acc(t_, " + x + ");";
-        }
         return c + " e" + std::to_string(id) + " = mf_dw_renorm(t_); }";
       }
       switch (n.op) {
@@ -2162,18 +2079,7 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
           o << ind << accref(j) << " += " << r << ";\n";
         else if (logprod[j] >= 0)
           o << ind << "mf_dw_logprod(lpm" << j << ", lpe" << j << ", " << eref(logprod[j]) << ");\n";
-        else if (!outsum[j].empty()) {
-          for (size_t m = 0; m < outsum[j].size(); m++) {
-            const Term& t = outsum[j][m];
-            const std::string x = t.minus ? "mf_dw_neg(" + eref(t.a) + ")" : eref(t.a);
-            if (fresh && m == 0)
-              o << ind << accref(j) << " = " << (t.b >= 0 ? "mf_dw_prod(" + x + ", " + eref(t.b) + ")" : x) << ";\n";
-            else if (t.b >= 0)
-              o << ind << "mf_dw_acc_mul(" << accref(j) << ", " << x << ", " << eref(t.b) << ");\n";
-            else
-              o << ind << "mf_dw_acc(" << accref(j) << ", " << x << ");\n";
-          }
-        } else if (fresh)
+        else if (fresh)
           o << ind << accref(j) << " = "
             << (fused[j].first >= 0 ? "mf_dw_prod(" + eref(fused[j].first) + ", " + eref(fused[j].second) + ")" : r)
             << ";\n";
@@ -2202,13 +2108,7 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
           deps = {logprod[j]};
         else if (ar == Ar::DW && logprod[j] >= 0)
           deps = {logprod[j]};
-        else if (ar == Ar::DW && !outsum[j].empty()) {
-          deps.clear();
-          for (const Term& t : outsum[j]) {
-            deps.push_back(t.a);
-            deps.push_back(t.b);
-          }
-        } else if (ar == Ar::DW && fused[j].first >= 0)
+        else if (ar == Ar::DW && fused[j].first >= 0)
           deps = {fused[j].first, fused[j].second};
         int at = -1;
         for (int d : deps)
