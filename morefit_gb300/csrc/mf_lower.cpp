@@ -2184,9 +2184,16 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
       for (int r = M; r > 0; r -= pick[r]) v.push_back(pick[r]);
       return v;
     }();
+    // Partials in shared memory: nothing of a chunk is loaded before the one
+    // before is done. ptxas otherwise loads all of them at once and spills, and
+    // callers split a Hessian that spills. Of a density linear in p + 1 columns,
+    // bytes a thread and one call at 1M events, without and with the barrier:
+    // p = 15 (120 outputs) 376 / 0, 194 / 161 us; p = 16 992 / 0, 229 / 196;
+    // p = 18 2144 / 568, 336 / 381; p = 20 2584 / 1304, 546 / 527.
     auto warp_reduce = [&](std::ostringstream& o) {  // into row `warp` of part[]
       int j0 = 0;
       for (int n : chunks) {
+        if (NREG < M) o << "  asm volatile(\"\" ::: \"memory\");\n";
         o << "  {\n    mf_dw v[" << n << "];\n";
         for (int c = 0; c < n; c++)
           o << "    v[" << c << "] = " << (j0 + c < M ? thread_dw(j0 + c) : "mf_dw_make(0.0f, 0.0f)") << ";\n";
