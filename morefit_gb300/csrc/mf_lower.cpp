@@ -2430,7 +2430,19 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
     // after the next are asked for in L2 (P-wave Hessian, 1M events 45.3 ->
     // 42.4 us, 3M 100 -> 93.8; a ring of three turns in shared memory, 42.7;
     // the gradients, 16 warps per SM and more, lose 3 us by either).
-    const bool lone_prefetch = !out.pipelined && NC > 0 && ar == Ar::DW && M <= kAccRegMax;
+    //
+    // "Fits" is two vectors of the columns, the partials, and 30 registers for
+    // the body (60 for Hessians, one event per turn) within 40 of the registers
+    // of a thread, 65536 over the block or 255: some spilled events cost less
+    // than the waits. Lone calls of 1M events, plain and prefetching (estimate
+    // at 256 threads): values of 31 columns 74 / 66 us (280), of 37 60 / 97
+    // (328), of 48 74 / 142 (416), of 64 134 / 1052 (544: 13 KB of spill);
+    // first evaluations of 31 columns 152 / 131, of 48 197 / 1506. The P-wave
+    // Hessian in blocks of 512 (168) spills 384 bytes, none with the plain loop.
+    auto fits = [&](int columns, int events) {
+      return 4 * columns * events + 2 * M + (events == 1 ? 60 : 30) < std::min(256, 65536 / out.block / 8 * 8) + 40;
+    };
+    const bool lone_prefetch = !out.pipelined && NC > 0 && ar == Ar::DW && M <= kAccRegMax && fits(NC, V);
     auto replace_all = [](std::string& t, const std::string& from, const std::string& to) {
       for (size_t p = t.find(from); p != std::string::npos; p = t.find(from, p + to.size())) t.replace(p, from.size(), to);
     };
@@ -2514,7 +2526,13 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
     // with the next columns' loads in flight and 36 without; a new dataset
     // with its precompute and first gradient 111.5 -> 98.9 us. For
     // gradient-sized kernels; Hessians are issue-bound and seldom first.
-    out.first = prep && pair && ar == Ar::DW && !st32 && !out.pipelined && NC > 0 && M <= 16;
+    // Only where the columns as they are, two vectors of them beside one of the
+    // prepared ones, fit as above.
+    std::set<int> raw_columns;
+    for (const auto& terms : fold.cols)
+      for (const auto& t : terms) raw_columns.insert(t.first);
+    out.first = prep && pair && ar == Ar::DW && !st32 && !out.pipelined && NC > 0 && M <= 16 &&
+                fits(std::max(NC, int(raw_columns.size())), V);
     if (out.first) {
       std::ostringstream first_work;
       block_work(first_work, false, true);
@@ -2537,7 +2555,7 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
     // vector of the columns and the partials take at most 56, which costs the
     // P-wave gradient 12 bytes of spill. Datasets in turn from HBM, 1M events:
     // 13.2 us an evaluation at the 86 registers it takes of itself, 11.0 at
-    // 80. The S+P wave (24 columns) would spill its events.
+    // 80. The S+P wave (16 columns) would spill its events.
     const bool three = ar == Ar::DW && out.block == 256 && NC > 1 && 2 * (NC * V + M) <= 56;
     s << "extern \"C\" __global__ void " << (three ? "__launch_bounds__(MF_BLOCK, 3) " : "MF_BOUNDS ") << out.entry
       << "_part(const " << DT
@@ -2640,8 +2658,8 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
     // and so: value of 1 toy 52 / 37 us, of 1000 144 / 112, of 4096 388 / 315;
     // F, gradient and Hessian of 1000 toys 311 / 304. Kernels whose partials
     // fill the registers (more than kAccRegMax outputs) and FP32 ones keep the
-    // plain loop (see lone_prefetch).
-    const bool seg_prefetch = ar == Ar::DW && M <= kAccRegMax;
+    // plain loop, and those whose events do not fit (see lone_prefetch).
+    const bool seg_prefetch = ar == Ar::DW && M <= kAccRegMax && fits(NC, 1);
     auto segment_work = [&](std::ostringstream& o) {
       auto load_event = [&](int k, const std::string& at) {
         return "__ldg(data + (mf_u64)" + std::to_string(k) + " * stride + first + " + at + ")";
