@@ -959,8 +959,13 @@ __device__ __forceinline__ mf_dw mf_dw_shfl_xor(mf_dw a, int o) {
 // (shared, complete for every thread on return). Thread (g, o) takes rows g,
 // g + MF_GRP, ... of output o, so that a warp's loads are contiguous and a
 // round of loads covers MF_Q rows per thread, added as a tree; then the MF_GRP
-// (at most 32) partials per output are added as a tree, by one thread (few) or
-// a warp. Measured as part of a lone launch, one thread per row and a shuffle
+// partials per output are added as a tree, by one thread (few) or a warp. All
+// of the block's threads take rows of a single output: its kernels are small,
+// so their full grids have up to 1216 rows, two and three rounds of loads for
+// 32 threads (1M events, FP32 values mass 22.1 -> 19.4 us, Crystal Ball 25.9 ->
+// 23.3, FP64 mass 26.0 -> 24.7). Two to seven outputs keep 32 threads each: the
+// mass gradient's registers (FP32 40 -> 42, FP64 48 -> 54) would cost a block
+// per SM. Measured as part of a lone launch, one thread per row and a shuffle
 // tree per output took 18 us of the P-wave Hessian's 54 (36 outputs, 152 rows,
 // ncu) and 100 of the S+P wave's 163 (105 outputs, 608 rows). A lone small
 // evaluation waits for every add in turn (about 60 cycles): trees instead of
@@ -1045,6 +1050,16 @@ __device__ __forceinline__ void mf_sum_rows(const float2* rows, unsigned nb, uns
   for (int j = threadIdx.x >> 5; j < MF_NOUT; j += MF_BLOCK / 32) {
     const int q = threadIdx.x & 31;
     mf_dw a = q < MF_GRP ? mf_dw_pair(part[q * MF_NOUT + j]) : mf_dw_make(0.0f, 0.0f);
+#if MF_GRP > 32
+    if (nb > 32u) {
+      mf_dw t[(MF_GRP + 31) / 32];
+#pragma unroll
+      for (int r = 0; r < (MF_GRP + 31) / 32; r++)
+        t[r] = q + 32 * r < MF_GRP ? mf_dw_pair(part[(q + 32 * r) * MF_NOUT + j]) : mf_dw_make(0.0f, 0.0f);
+      mf_tree_sum(t);
+      a = t[0];
+    }
+#endif
 #pragma unroll
     for (int w = MF_GRP > 16 ? 16 : 8; w > 0; w >>= 1) a = mf_dw_add(a, mf_dw_shfl_xor(a, w));
     if (q == 0) sums[j] = make_float2(a.h, a.l);
@@ -1417,12 +1432,13 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
   s << "#define MF_NREG " << NREG << "\n";
   // launch bounds of the event-loop entries
   s << "#define MF_BOUNDS __launch_bounds__(MF_BLOCK)\n";
-  // combine of block partial rows: MF_GRP threads (a warp's lanes at most) share an output's rows, each
-  // with MF_Q loads in flight; kernels of many outputs, whose grids of small
-  // blocks leave hundreds of rows, combine them in groups of MF_ROWS blocks first
-  const int grp = std::max(1, std::min(32, out.block / M));
+  // combine of block partial rows: MF_GRP threads (a warp's lanes at most, the
+  // whole block for a single output) share an output's rows, each with MF_Q
+  // loads in flight; kernels of many outputs, whose grids of small blocks leave
+  // hundreds of rows, combine them in groups of MF_ROWS blocks first
+  const int grp = M == 1 ? out.block : std::max(1, std::min(32, out.block / M));
   int q = 2;  // a power of two: the rows of a round are added as a tree
-  while (q < 16 && q * grp < 608) q *= 2;
+  while (q < 16 && q * grp < (M == 1 ? 8 * 152 : 608)) q *= 2;
   s << "#define MF_GRP " << grp << "\n#define MF_Q " << q << "\n";
   s << "#define MF_ROWS " << (M > kAccRegMax ? kCombineRows : 0) << "\n";
   // shared scratch of the block reduction (a row per warp) and the combine (MF_GRP rows)
