@@ -2220,7 +2220,27 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
         j0 += n;
       }
     };
+    // Up to eight outputs (256 threads) of FP32 kernels, a warp each: through
+    // shared memory, so that a block does M warps' sums instead of M outputs'
+    // butterflies in each of its eight warps (1370 instructions for 5 outputs,
+    // 1070 so); batched gradients of 250k events, FP32 mass 2.23 -> 2.02 us an
+    // evaluation, weighted 2.38 -> 2.18. Double-float kernels share the
+    // butterfly's order with their _batch entry.
+    const bool staged = (ar == Ar::F32 || ar == Ar::F32S) && M <= out.block / 32 && M * out.block <= 2048;  // 16 KB
     auto block_reduce = [&](std::ostringstream& o) {
+      if (staged) {
+        o << "  __shared__ float2 mf_stage[MF_NOUT][MF_BLOCK];\n"
+          << "  __shared__ float2 mf_part[MF_PART];\n  __shared__ float2 mf_blk[MF_NOUT];\n"
+          << "  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;\n";
+        for (int j = 0; j < M; j++)
+          o << "  { const mf_dw t = " << thread_dw(j) << "; mf_stage[" << j << "][threadIdx.x] = make_float2(t.h, t.l); }\n";
+        o << "  __syncthreads();\n  if (warp < MF_NOUT) {\n    mf_dw t[MF_BLOCK / 32];\n"
+          << "#pragma unroll\n    for (int k = 0; k < MF_BLOCK / 32; k++) t[k] = mf_dw_pair(mf_stage[warp][lane + 32 * k]);\n"
+          << "    mf_tree_sum(t);\n"
+          << "#pragma unroll\n    for (int o = 16; o > 0; o >>= 1) t[0] = mf_dw_add(t[0], mf_dw_shfl_xor(t[0], o));\n"
+          << "    if (lane == 0) mf_blk[warp] = make_float2(t[0].h, t[0].l);\n  }\n  __syncthreads();\n";
+        return;
+      }
       o << "  __shared__ float2 mf_part[MF_PART];\n  __shared__ float2 mf_blk[MF_NOUT];\n"
         << "  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;\n  float2* const part = mf_part;\n";
       warp_reduce(o);
