@@ -1506,7 +1506,17 @@ struct BatchJob {
 // events 149 / 51, 20k 148 / 76, 50k 152 / 100, 100k 166 / 149, 150k 212 /
 // 188; its value 100k 147 / 100; mass gradient 1k 178 / 70, 50k 172 / 132,
 // 150k 260 / 265; S+P gradient 20k 180 / 133, 50k 191 / 193.
+//
+// Kernels that read more than 48 values an event vector keep them in up to 255
+// registers there, one block per SM, where their launches of their own keep
+// two and three: such evaluations go up to 25 values per SM and block. 8 and 64
+// points, a launch each against _batch (us): 25 columns, gradient 24k events 33
+// / 31, 122 / 88, 60k 40 / 47, 173 / 191; 48 columns, value 16k 33 / 31, 122 /
+// 100, 24k 35 / 37, 127 / 132, 60k 44 / 57, 217 / 243; 64 columns, value 8k 34
+// / 29, 122 / 90, 16k 35 / 38, 122 / 135, 60k 62 / 85, 339 / 398.
 bool batch_fits(const mf_kernel* k, int maxgrid) {
+  const size_t values = k->lowered.used_inputs.size() * size_t(k->lowered.vec);
+  if (values > 48 && size_t(maxgrid) * values > size_t(k->ctx->num_sms) * 25) return false;
   return k->fn_batch && maxgrid < k->ctx->num_sms * k->blocks_per_sm;
 }
 
