@@ -2205,11 +2205,13 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
     // callers split a Hessian that spills. Of a density linear in p + 1 columns,
     // bytes a thread and one call at 1M events, without and with the barrier:
     // p = 15 (120 outputs) 376 / 0, 194 / 161 us; p = 16 992 / 0, 229 / 196;
-    // p = 18 2144 / 568, 336 / 381; p = 20 2584 / 1304, 546 / 527.
+    // p = 18 2144 / 568, 336 / 381; p = 20 2584 / 1304, 546 / 527. Up to 32
+    // partials in registers there is no spill either way: the S+P wave's 105
+    // outputs (25) take 71.5 / 76.3 us at 333333 events, 152 / 148 at 1M.
     auto warp_reduce = [&](std::ostringstream& o) {  // into row `warp` of part[]
       int j0 = 0;
       for (int n : chunks) {
-        if (NREG < M) o << "  asm volatile(\"\" ::: \"memory\");\n";
+        if (NREG < M && NREG > 32) o << "  asm volatile(\"\" ::: \"memory\");\n";
         o << "  {\n    mf_dw v[" << n << "];\n";
         for (int c = 0; c < n; c++)
           o << "    v[" << c << "] = " << (j0 + c < M ? thread_dw(j0 + c) : "mf_dw_make(0.0f, 0.0f)") << ";\n";
@@ -2592,6 +2594,8 @@ LoweredKernel lower(const std::string& name, Kind kind, Elem elem, const std::ve
     // P-wave gradient 12 bytes of spill. Datasets in turn from HBM, 1M events:
     // 13.2 us an evaluation at the 86 registers it takes of itself, 11.0 at
     // 80. The S+P wave (16 columns) would spill its events.
+    // Kernels of one column take fewer than 80 of themselves, and the bound raises
+    // them (mass value 48 -> 56, gradient 48 -> 64): a block per SM less.
     const bool three = ar == Ar::DW && out.block == 256 && NC > 1 && 2 * (NC * V + M) <= 56;
     s << "extern \"C\" __global__ void " << (three ? "__launch_bounds__(MF_BLOCK, 3) " : "MF_BOUNDS ") << out.entry
       << "_part(const " << DT
